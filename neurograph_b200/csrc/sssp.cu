@@ -235,8 +235,8 @@ int launch_tiles(ngx_graph* g, const ngx_apsp_opts* opts, int tile_mode, const T
     const int width = batched ? kTile : 1;
     const int64_t num_tiles = batched ? job.num_items : job.num_sources;
     const int block = opts->block_threads > 0 ? opts->block_threads : (batched ? kBatchedDefaultBlock : 512);
-    const size_t acc_bytes = static_cast<size_t>(2) * (batched ? kTile : kPlainWarpsMax) * kAccDigits * 8;
-    const size_t smem = acc_bytes + static_cast<size_t>(hist_bins) * 4;
+    const size_t fixed_smem = batched ? sizeof(TileSmem) : static_cast<size_t>(2) * kPlainWarpsMax * kAccDigits * 8;
+    const size_t smem = fixed_smem + static_cast<size_t>(hist_bins) * 4;
     if (!batched && job.num_graphs != 1) {
         return fail(NGX_UNSUPPORTED, "the plain form runs one graph at a time");
     }
@@ -315,9 +315,7 @@ int launch_tiles(ngx_graph* g, const ngx_apsp_opts* opts, int tile_mode, const T
     p.ws_dist = reinterpret_cast<unsigned long long*>(ws);
     ws += static_cast<size_t>(slots) * n * width * 8;
     p.ws_pend = reinterpret_cast<uint32_t*>(ws);
-    ws += static_cast<size_t>(slots) * 2 * n * 4;
-    p.ws_far = reinterpret_cast<uint32_t*>(ws);
-    ws += static_cast<size_t>(slots) * n * 4;
+    ws += static_cast<size_t>(slots) * 3 * n * 4;
     p.ws_queue = reinterpret_cast<int32_t*>(ws);
     ws += static_cast<size_t>(slots) * 2 * n * 4;
     p.ws_stamp = reinterpret_cast<uint32_t*>(ws);
@@ -461,7 +459,7 @@ int launch_apsp_in_workspace(ngx_graph* g, const ngx_apsp_opts* opts, const Tile
     if (job.num_items == 0) {
         return NGX_OK;
     }
-    const size_t smem = static_cast<size_t>(2) * kTile * kAccDigits * 8 + static_cast<size_t>(hist_bins) * 4;
+    const size_t smem = sizeof(TileSmem) + static_cast<size_t>(hist_bins) * 4;
     NGX_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     int per_sm = 0;
     NGX_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, smem));
@@ -498,9 +496,7 @@ int launch_apsp_in_workspace(ngx_graph* g, const ngx_apsp_opts* opts, const Tile
     p.ws_dist = reinterpret_cast<unsigned long long*>(w);
     w += static_cast<size_t>(slots) * n * kTile * 8;
     p.ws_pend = reinterpret_cast<uint32_t*>(w);
-    w += static_cast<size_t>(slots) * 2 * n * 4;
-    p.ws_far = reinterpret_cast<uint32_t*>(w);
-    w += static_cast<size_t>(slots) * n * 4;
+    w += static_cast<size_t>(slots) * 3 * n * 4;
     p.ws_queue = reinterpret_cast<int32_t*>(w);
     w += static_cast<size_t>(slots) * 2 * n * 4;
     p.ws_stamp = reinterpret_cast<uint32_t*>(w);

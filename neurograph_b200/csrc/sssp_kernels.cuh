@@ -70,10 +70,9 @@ struct SsspParams {
     const volatile int* abort_flag;
     // workspace, carved per slot (blockIdx.x)
     unsigned long long* ws_dist;   // slots * n * width (width = kTile batched, 1 plain)
-    uint32_t* ws_pend;             // slots * 2n
-    uint32_t* ws_far;              // slots * n
+    uint32_t* ws_pend;             // slots * 3n: two pending masks (alternating by iteration parity) and the far marks
     int32_t* ws_queue;             // slots * 2n
-    uint32_t* ws_stamp;            // slots * n
+    uint32_t* ws_stamp;            // slots * n; tile kernel: the distance phase's bound[], then the DAG passes' stamps
     // reach lists (graphs of several strongly connected components; nullptr otherwise): per vertex the tile's
     // sources that reached it, and the list of the vertices reached, so that per-tile passes visit only those
     uint32_t* ws_reach;            // slots * n
@@ -173,61 +172,148 @@ struct Reach {
     }
 };
 
-// The relaxations of kUnroll (arc, source) pairs per lane, their loads done: pair u relaxes d[x[u]][src[u]] with nd[u]
-// (cur[u] = the distance read before). The atomic minima are issued back to back and waited for together (APSP mode:
-// not waited for at all), then the marks; see batched_expand for what each mode does with an improvement.
+// Arcs of one vertex that batched_expand filters together (four per lane).
+constexpr int kArcBlock = 128;
+
+// One queue entry a warp has taken: a vertex, its pending sources, its first arc and out-degree.
+struct __align__(16) QueueEntry {
+    int v;
+    uint32_t mask;
+    uint32_t beg;
+    int deg;
+};
+
+// A warp's scratch in the distance phase. Keeping the chunk's entries here and the pointers in ExpandArgs leaves the
+// registers to the reads in flight: with all of it in registers the compiler spilled the records just read, so that each
+// read was waited for before the next was issued (measured on the 100,000-vertex connectome, 16 warps x 2 CTAs per SM:
+// 3700 cycles for a vertex's four arc reads per lane, 1500 without spills).
+struct WarpScratch {
+    Arc kept[kArcBlock];     // arcs that passed the filter (batched_expand); id = position in the row
+    QueueEntry entry[32];    // the chunk
+    int rank[32];            // pending sources by rank (batched_expand), entry << 5 | source (packed_expand)
+};
+
+// A warp's share of the run's work counters.
+struct WarpWork {
+    unsigned long long expansions;
+    unsigned long long lane_expansions;
+};
+
+constexpr int kMaxWarps = 16;
+constexpr int kAccBytes = 2 * kTile * kAccDigits * 8;
+
+// Per-tile arguments of the distance phase, in shared memory.
+struct ExpandArgs {
+    const Arc* arcs;
+    const int64_t* row_ptr;
+    unsigned long long* dist;
+    uint32_t* marks;              // pending masks of even and odd iterations, far marks: three times n_slot words
+    int32_t* queue;               // two queues of n_slot entries
+    uint8_t* bound;
+    int* grab;
+    unsigned long long* pred_key;
+    unsigned long long* last;
+    uint32_t* tie;
+    Reach reach;
+    uint32_t n_slot;
+    int nsrc;
+    int bound_base;
+    int group_warps;
+};
+
+// Dynamic shared memory of the tile kernel, before the histogram. The distance phase's warp scratch overlays the
+// epilogue's accumulators (2 x kTile x kAccDigits words, zero outside the distance phase) and, after them, the scan
+// partials of the DAG phase.
+struct TileSmem {
+    WarpScratch warp[kMaxWarps];
+    WarpWork work[kMaxWarps];
+    ExpandArgs args;
+    TileShared ctl;
+};
+static_assert(sizeof(WarpScratch) * kMaxWarps >= kAccBytes + (512 + 3) * 8, "accumulators and scan partials fit in the warp scratch");
+static_assert(sizeof(TileSmem) % 16 == 0, "the histogram follows");
+
+// The relaxations of kUnroll arcs by this lane's source, their loads done: arc u relaxes d[x[u]][src] with nd[u] (cur[u] =
+// the distance read before); an infinite nd[u] relaxes nothing. The atomic minima are issued back to back and waited for
+// together (APSP mode: not waited for at all), then the marks; see batched_expand for what each mode does with an
+// improvement. dist_s points at the source's column.
 template <int kUnroll, bool kTrack, bool kReach>
-__device__ __forceinline__ void relax_pairs(const int (&x)[kUnroll], const int (&src)[kUnroll], const double (&nd)[kUnroll],
-                                            unsigned long long (&cur)[kUnroll], const uint32_t (&eidx)[kUnroll], const bool (&valid)[kUnroll],
-                                            unsigned long long* __restrict__ dist, uint32_t* pend_nxt, uint32_t* far, double theta,
-                                            unsigned long long* pred_key, uint32_t* tie, const Reach& reach) {
-    // the atomic minima (cur[u] becomes the old value where it is waited for)
+__device__ __forceinline__ void relax_lane(const int (&x)[kUnroll], int src, const double (&nd)[kUnroll], unsigned long long (&cur)[kUnroll],
+                                           const uint32_t (&eidx)[kUnroll], unsigned long long* dist_s, const TileSmem& sh) {
     bool tried[kUnroll];
 #pragma unroll
     for (int u = 0; u < kUnroll; ++u) {
         const unsigned long long nb = static_cast<unsigned long long>(__double_as_longlong(nd[u]));
-        tried[u] = valid[u] && nb < cur[u];
+        tried[u] = nb < cur[u] || (kTrack && nb == cur[u] && nb != kInfBits);
         if (tried[u]) {
             if constexpr (kTrack) {
-                cur[u] = atomicMin(&dist[static_cast<int64_t>(x[u]) * kTile + src[u]], nb);
+                // an equal value is a tie already (the minimum would return it unchanged)
+                cur[u] = nb < cur[u] ? atomicMin(&dist_s[static_cast<int64_t>(x[u]) * kTile], nb) : nb;
             } else {
-                atomicMin(&dist[static_cast<int64_t>(x[u]) * kTile + src[u]], nb);
+                atomicMin(&dist_s[static_cast<int64_t>(x[u]) * kTile], nb);
             }
         }
     }
+    const uint32_t bit = 1u << src;
 #pragma unroll
     for (int u = 0; u < kUnroll; ++u) {
-        const unsigned long long nb = static_cast<unsigned long long>(__double_as_longlong(nd[u]));
         if (tried[u]) {
+            const unsigned long long nb = static_cast<unsigned long long>(__double_as_longlong(nd[u]));
             const unsigned long long old = cur[u];
             if constexpr (kTrack) {
                 if (nb < old) {
-                    atomicMin(&pred_key[static_cast<int64_t>(x[u]) * kTile + src[u]], ((nb >> 32) << 32) | eidx[u]);
+                    atomicMin(&sh.args.pred_key[static_cast<int64_t>(x[u]) * kTile + src], ((nb >> 32) << 32) | eidx[u]);
                 } else if (nb == old) {
-                    atomicOr(&tie[x[u]], 1u << src[u]);
+                    atomicOr(&sh.args.tie[x[u]], bit);
                 }
             }
-            if (nb < old) {
-                const uint32_t bit = 1u << src[u];
+            if (!kTrack || nb < old) {
                 if (kReach && old == kInfBits) {
-                    reach.add(x[u], bit);  // the first distance of (x, s): x joins the tile's reached vertices
+                    sh.args.reach.add(x[u], bit);  // the first distance of (x, s): x joins the tile's reached vertices
                 }
-                if (nd[u] < theta) {
-                    atomicOr(&pend_nxt[x[u]], bit);
-                } else {
-                    atomicOr(&far[x[u]], bit);
-                }
+                const uint32_t which = nd[u] < sh.ctl.theta ? static_cast<uint32_t>(sh.ctl.cur ^ 1) : 2u;
+                atomicOr(&sh.args.marks[static_cast<size_t>(which) * sh.args.n_slot + static_cast<uint32_t>(x[u])], bit);
             }
-        } else if (kTrack && valid[u] && nb == cur[u]) {
-            atomicOr(&tie[x[u]], 1u << src[u]);
         }
     }
 }
 
 // ------------------------------------------------------------------------------------------ batched form
-// Expands vertex v for the k sources pending on it. The deg(v) x k (arc, source) pairs are spread over the 32 lanes:
-// pair p = 32 i + lane takes arc p / k and the (p % k)-th pending source, so no lane idles when few sources are
-// pending, and when all 32 are, every iteration reads one whole distance row d[x][0..31] (256 contiguous bytes).
+// A bound is one byte, so that the bounds of 100,000 vertices fit in a fair part of an SM's L1: the exponent and five
+// mantissa bits of the row maximum (steps of 3 %), counted from a quarter of the bucket width (8 octaves: up to 64
+// bucket widths). kNoBound stands for unknown and for anything larger. Truncation keeps the order of non-negative
+// doubles, so key(a) > key(b) implies a > b.
+constexpr int kNoBound = 255;
+__device__ __forceinline__ int bound_key(uint32_t hi, int base) { return static_cast<int>(hi >> 15) - base; }
+// Read through L1 (unlike the distances): the tile's group barriers order a reader after the reset of the tile before,
+// and within a tile a stale bound is only weaker. volatile: not moved across a barrier.
+__device__ __forceinline__ int ld_bound(const uint8_t* p) {
+    uint32_t v;
+    asm volatile("ld.global.L1::evict_last.u8 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return static_cast<int>(v);
+}
+// An arc record that this SM is not expected to read again soon: it does not displace the bounds from L1.
+__device__ __forceinline__ Arc ldg_arc_once(const Arc* p) {
+    int4 v;
+    asm("ld.global.nc.L1::no_allocate.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return Arc{ v.x, v.y, __hiloint2double(v.w, v.z) };
+}
+
+// Vertices with fewer arcs are not filtered: at out-degree 6 (integer weights) 84 % of the arcs pass, at 20 and more
+// (log-normal and integer weights) 36-60 % of the (arc, source) pairs remain.
+constexpr int kFilterDegree = 16;
+
+// Expands vertex v for the k sources pending on it, in two steps.
+// 1. The arc filter. bound[x] is an upper bound of every d[x][s] of the tile: each expansion of x reads its whole
+//    distance row (256 contiguous bytes) and stores the key of the row's maximum. Distances only decrease, so a bound
+//    never becomes false and a stale one is only weaker. With d_min the smallest pending distance of v, an arc (v, x)
+//    whose fl(d_min + len) has a larger key than bound[x] is longer than every final d[x][s]: its relaxations can
+//    neither improve nor tie with any of them (fl is monotone), so the arc is dropped for a one-byte read instead of k
+//    8-byte reads.
+// 2. The pair loop. Each lane keeps one pending source for all its pairs (lane mod k' of them, k' = k rounded up to a
+//    power of two) and takes every (32 / k')-th kept arc, so a pair costs one shared-memory read, an addition, a distance
+//    read and a comparison; up to half of the lanes idle when k is just above a power of two, which is cheaper than
+//    finding each pair's arc and source anew (three shuffles and a carry per pair).
 // An improvement below theta sets the pair's bit in pend_nxt (the next iteration's queue is compacted from those
 // masks after the iteration), one at or above theta its far mark. The kUnroll relaxations of a lane are issued back
 // to back and waited for together.
@@ -242,188 +328,164 @@ __device__ __forceinline__ void relax_pairs(const int (&x)[kUnroll], const int (
 // arc in its key (the DAG count pass checks it). For that, no (v, s) may be expanded twice with one distance (the
 // repeat would look like a tie): last[v][s] keeps the distance of the latest expansion, and sources whose distance has
 // not changed since are dropped from the next.
-// The caller has taken v's pending mask (amask, non-zero), cleared it and v's superseded far marks, and read its row
-// offsets (beg, deg): see expand_queue.
+// The caller has taken v's pending mask (entry.mask, non-zero) and cleared it and v's superseded far marks: see
+// expand_queue. Lanes >= nsrc hold no source.
 template <int kUnroll, bool kTrack, bool kReach>
-__device__ __forceinline__ void batched_expand(const DeviceCsr& g, int v, uint32_t amask, int64_t beg, int deg, int lane,
-                                               unsigned long long* __restrict__ dist, uint32_t* pend_nxt, uint32_t* far, double theta,
-                                               unsigned long long& expansions, unsigned long long& lane_expansions, unsigned long long* pred_key,
-                                               uint32_t* tie, unsigned long long* last, const Reach& reach) {
-    const uint32_t amask0 = amask;
-    int k = __popc(amask);
-    // lane r < k holds the r-th pending source and its distance to v
-    int rank_src = lane < k ? static_cast<int>(__fns(amask, 0, lane + 1)) : 0;
-    unsigned long long rank_bits = __ldcg(&dist[static_cast<int64_t>(v) * kTile + rank_src]);
+__device__ __forceinline__ void batched_expand(TileSmem& sh, WarpScratch& w, WarpWork& work, int j, int lane) {
+    const QueueEntry entry = w.entry[j];
+    uint32_t amask = entry.mask;
+    unsigned long long* const dist = sh.args.dist;
+    const Arc* const arcs = sh.args.arcs + entry.beg;
+    const int64_t vrow = static_cast<int64_t>(entry.v) * kTile + lane;
+    const unsigned long long row_bits = __ldcg(&dist[vrow]);
+    const uint32_t row_hi = static_cast<uint32_t>(row_bits >> 32);
     if constexpr (kTrack) {
-        unsigned long long* const slot = &last[static_cast<int64_t>(v) * kTile + rank_src];
-        const bool repeat = lane < k && __ldcg(slot) == rank_bits;
-        if (lane < k && !repeat) {
-            *slot = rank_bits;
+        unsigned long long* const last = sh.args.last;
+        const bool pending = (amask >> lane) & 1u;
+        const bool repeat = pending && __ldcg(&last[vrow]) == row_bits;
+        if (pending && !repeat) {
+            last[vrow] = row_bits;
         }
-        const uint32_t drop = __reduce_or_sync(kFullMask, repeat ? (1u << rank_src) : 0u);
-        if (drop != 0u) {
-            amask &= ~drop;
-            if (amask == 0u) {
-                return;
-            }
-            // re-rank the remaining sources; their distances come from the lanes that read them
-            const int new_k = __popc(amask);
-            const int src_new = lane < new_k ? static_cast<int>(__fns(amask, 0, lane + 1)) : 0;
-            const int old_rank = __popc(amask0 & ((1u << src_new) - 1u));
-            rank_bits = __shfl_sync(kFullMask, rank_bits, old_rank);
-            rank_src = src_new;
-            k = new_k;
-        }
+        amask &= ~__ballot_sync(kFullMask, repeat);
     }
-    expansions += 1;
-    lane_expansions += static_cast<unsigned long long>(k);
-    const double rank_dv = __longlong_as_double(static_cast<long long>(rank_bits));
-    const Arc* arcs = g.arcs + beg;
-    // v's arc records (16 B each) into L1 ahead of the pair loop, one 128-byte line per lane
-    if (lane * 8 < deg) {
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(arcs + lane * 8));
+    const int bound_base = sh.args.bound_base;
+    const uint32_t row_max = __reduce_max_sync(kFullMask, lane < sh.args.nsrc ? row_hi : 0u);
+    const int max_key = bound_key(row_max, bound_base);
+    if (lane == 0 && max_key < kNoBound) {
+        sh.args.bound[entry.v] = static_cast<uint8_t>(max_key > 0 ? max_key : 0);
     }
-    // position of this lane's first pair, and the per-iteration advance of 32 pairs
-    int a = lane / k;
-    int r = lane - a * k;
-    const int step_a = 32 / k;
-    const int step_r = 32 - step_a * k;
-    const int64_t total = static_cast<int64_t>(deg) * k;
-    for (int64_t p0 = 0; p0 < total; p0 += 32 * kUnroll) {
-        int x[kUnroll];
-        int src[kUnroll];
-        double nd[kUnroll];
-        unsigned long long cur[kUnroll];
-        uint32_t eidx[kUnroll];
-        bool valid[kUnroll];
+    if (amask == 0u) {
+        return;
+    }
+    const uint32_t min_hi = __reduce_min_sync(kFullMask, ((amask >> lane) & 1u) != 0u ? row_hi : 0xFFFFFFFFu);
+    const double d_min = __hiloint2double(static_cast<int>(min_hi), 0);  // at most every pending distance
+    const int k = __popc(amask);
+    // this lane's source: the r-th pending one, r = lane mod k rounded up to a power of two (no source for r >= k), and
+    // its distance to v
+    if ((amask >> lane) & 1u) {
+        w.rank[__popc(amask & lanemask_lt())] = lane;
+    }
+    if (lane == 0) {
+        work.expansions += 1ull;
+        work.lane_expansions += static_cast<unsigned long long>(k);
+    }
+    __syncwarp();
+    const int log_k = 32 - __clz(k - 1);
+    const int r = lane & ((1 << log_k) - 1);
+    const int src = r < k ? w.rank[r] : 0;
+    const double dvs = __longlong_as_double(static_cast<long long>(__shfl_sync(kFullMask, row_bits, src)));
+    unsigned long long* const dist_s = dist + src;
+    const int first_a = r < k ? lane >> log_k : kArcBlock;  // this lane's first kept arc of a block
+    const int step_a = 32 >> log_k;
+    const bool filter = entry.deg >= kFilterDegree;
+    for (int a0 = 0; a0 < entry.deg; a0 += kArcBlock) {
+        int kept = 0;
+        {
+            Arc arc[kArcBlock / 32];
+            int ub[kArcBlock / 32];
+            const uint8_t* const bound = sh.args.bound;
 #pragma unroll
-        for (int u = 0; u < kUnroll; ++u) {
-            valid[u] = a < deg;
-            eidx[u] = static_cast<uint32_t>(beg + a);
-            src[u] = __shfl_sync(kFullMask, rank_src, r);
-            const double dvs = __shfl_sync(kFullMask, rank_dv, r);
-            x[u] = 0;
-            nd[u] = 0.0;
-            cur[u] = 0ull;
-            if (valid[u]) {
-                const Arc arc = ldg_arc(&arcs[a]);
-                x[u] = arc.col;
-                nd[u] = __dadd_rn(dvs, arc.len);
-                cur[u] = __ldcg(&dist[static_cast<int64_t>(x[u]) * kTile + src[u]]);
+            for (int u = 0; u < kArcBlock / 32; ++u) {
+                // a lane past the last arc reads the last one again and keeps nothing
+                const int i = a0 + u * 32 + lane;
+                arc[u] = ldg_arc_once(&arcs[i < entry.deg ? i : entry.deg - 1]);
             }
-            a += step_a;
-            r += step_r;
-            if (r >= k) {
-                r -= k;
-                a += 1;
+#pragma unroll
+            for (int u = 0; u < kArcBlock / 32; ++u) {
+                ub[u] = filter ? ld_bound(&bound[arc[u].col]) : kNoBound;
+            }
+#pragma unroll
+            for (int u = 0; u < kArcBlock / 32; ++u) {
+                const int i = a0 + u * 32 + lane;
+                const int key = bound_key(static_cast<uint32_t>(__double2hiint(__dadd_rn(d_min, arc[u].len))), bound_base);
+                const bool keep = i < entry.deg && (key <= ub[u] || ub[u] == kNoBound);
+                const unsigned bal = __ballot_sync(kFullMask, keep);
+                if (keep) {
+                    w.kept[kept + __popc(bal & lanemask_lt())] = Arc{ arc[u].col, i, arc[u].len };
+                }
+                kept += __popc(bal);
             }
         }
-        relax_pairs<kUnroll, kTrack, kReach>(x, src, nd, cur, eidx, valid, dist, pend_nxt, far, theta, pred_key, tie, reach);
+        __syncwarp();
+        int a = first_a;
+        for (int a_warp = 0; a_warp < kept; a_warp += step_a * kUnroll) {
+            int x[kUnroll];
+            double nd[kUnroll];
+            unsigned long long cur[kUnroll];
+            uint32_t eidx[kUnroll];
+#pragma unroll
+            for (int u = 0; u < kUnroll; ++u) {
+                // a lane without a pair reads the first kept arc's and relaxes nothing
+                const Arc kept_arc = w.kept[a < kept ? a : 0];
+                x[u] = kept_arc.col;
+                eidx[u] = entry.beg + static_cast<uint32_t>(kept_arc.id);
+                nd[u] = a < kept ? __dadd_rn(dvs, kept_arc.len) : INFINITY;
+                cur[u] = __ldcg(&dist_s[static_cast<int64_t>(x[u]) * kTile]);
+                a += step_a;
+            }
+            relax_lane<kUnroll, kTrack, kReach>(x, src, nd, cur, eidx, dist_s, sh);
+        }
+        __syncwarp();  // the next block of arcs (the next vertex) overwrites kept (and rank)
     }
 }
 
-// Queue entries with fewer (arc, pending source) pairs than this fill less than one iteration of batched_expand's
-// pair loop (32 lanes x 4 pairs at the library's unroll); consecutive ones are expanded together by packed_expand,
-// whose division of a pair index by the entry's source count is exact only below 2^7 pairs per entry.
-constexpr int kPackPairs = 128;
-static_assert(kPackPairs <= 128, "packed_expand divides pair indices below 2^7 by a 16-bit reciprocal");
+// Queue entries with fewer (arc, pending source) pairs than this leave most of a warp idle in batched_expand (32 lanes,
+// several arcs per lane in flight); consecutive ones are expanded together by packed_expand.
+#ifndef NGX_PACK_PAIRS
+#define NGX_PACK_PAIRS 64
+#endif
+constexpr int kPackPairs = NGX_PACK_PAIRS;
 
-// Expands a group of m small queue entries together, so that one iteration of the pair loop serves several vertices.
-// Lane i < m holds entry i: its vertex gv, pending mask gmask (non-zero), first arc gbeg and out-degree gdeg; the
-// entries have at most 32 pending sources in all. Lane t then holds the t-th (entry, pending source) of the group and
-// that source's distance to the entry's vertex, and the group's pairs are dealt to the lanes entry after entry: pair
-// q of entry i (0 <= q < k_i deg_i) is arc q / k_i with the (q % k_i)-th pending source, as in batched_expand. The
-// relaxations, the repeat check of the DAG modes (a repeated (vertex, source) only drops its own pairs here) and the
-// counters are batched_expand's.
+// Expands a group of m small queue entries together: w.rank[t], t < ktot <= 32, names the t-th (entry, pending source) of
+// the group. Lane t takes it and walks its entry's arcs, kUnroll at a time: the lanes of an entry read the same arc
+// records and neighbouring distances of the same rows, no lane needs to find its pairs, and the group takes as long as
+// its entry with the most arcs. The relaxations, the repeat check of the DAG modes and the counters are
+// batched_expand's; the arcs are not filtered (a bound read per arc would cost as much as the few distance reads it
+// saves).
 template <int kUnroll, bool kTrack, bool kReach>
-__device__ __forceinline__ void packed_expand(const DeviceCsr& g, int m, int gv, uint32_t gmask, int64_t gbeg, int gdeg, int lane,
-                                              unsigned long long* __restrict__ dist, uint32_t* pend_nxt, uint32_t* far, double theta,
-                                              unsigned long long& expansions, unsigned long long& lane_expansions, unsigned long long* pred_key,
-                                              uint32_t* tie, unsigned long long* last, const Reach& reach) {
-    // per entry (lane i < m): pending sources k_i, pairs, offsets of its ranks and pairs in the group, 16-bit reciprocal
-    const int ki = lane < m ? __popc(gmask) : 0;
-    const int pi = lane < m ? ki * gdeg : 0;
-    int kinc = ki, pinc = pi;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const int ku = __shfl_up_sync(kFullMask, kinc, off);
-        const int pu = __shfl_up_sync(kFullMask, pinc, off);
-        if (lane >= off) {
-            kinc += ku;
-            pinc += pu;
-        }
-    }
-    const int ri = kinc - ki;
-    const int si = pinc - pi;
-    const int ktot = __shfl_sync(kFullMask, kinc, 31);
-    const int ptot = __shfl_sync(kFullMask, pinc, 31);
-    // floor(q / k) = (q * ceil(2^16 / k)) >> 16 exactly for q < 2^7 and k <= 32
-    const int mgi = lane < m ? (65536 + ki - 1) / ki : 0;
-    // lane t < ktot: its entry (the number of entries whose ranks start at or below t, minus one) and rank
-    const unsigned starts = __reduce_or_sync(kFullMask, lane < m ? (1u << ri) : 0u);
-    const int et = lane < ktot ? __popc(starts & ((2u << lane) - 1u)) - 1 : 0;
-    const uint32_t emask = __shfl_sync(kFullMask, gmask, et);
-    const int ev = __shfl_sync(kFullMask, gv, et);
-    const int er = __shfl_sync(kFullMask, ri, et);
-    const int rank_src = lane < ktot ? static_cast<int>(__fns(emask, 0, lane - er + 1)) : 0;
-    const unsigned long long rank_bits = __ldcg(&dist[static_cast<int64_t>(ev) * kTile + rank_src]);
-    bool rank_ok = lane < ktot;
+__device__ __forceinline__ void packed_expand(TileSmem& sh, WarpScratch& w, WarpWork& work, int m, int ktot, int lane) {
+    const int code = w.rank[lane < ktot ? lane : 0];
+    const int src = code & 31;
+    const QueueEntry entry = w.entry[code >> 5];
+    const int64_t vrow = static_cast<int64_t>(entry.v) * kTile + src;
+    unsigned long long* const dist_s = sh.args.dist + src;
+    const unsigned long long v_bits = __ldcg(&dist_s[static_cast<int64_t>(entry.v) * kTile]);
+    bool ok = lane < ktot;
     if constexpr (kTrack) {
-        unsigned long long* const slot = &last[static_cast<int64_t>(ev) * kTile + rank_src];
-        if (rank_ok && __ldcg(slot) == rank_bits) {
-            rank_ok = false;  // expanded with this distance already
-        } else if (rank_ok) {
-            *slot = rank_bits;
+        unsigned long long* const last = sh.args.last;
+        if (ok && __ldcg(&last[vrow]) == v_bits) {
+            ok = false;  // expanded with this distance already
+        } else if (ok) {
+            last[vrow] = v_bits;
         }
     }
-    const unsigned ok_mask = __ballot_sync(kFullMask, rank_ok);
-    if (ok_mask == 0u) {
-        return;
+    const unsigned ok_mask = __ballot_sync(kFullMask, ok);
+    if (lane == 0 && ok_mask != 0u) {
+        work.expansions += static_cast<unsigned long long>(m);
+        work.lane_expansions += static_cast<unsigned long long>(__popc(ok_mask));
     }
-    expansions += static_cast<unsigned long long>(m);
-    lane_expansions += static_cast<unsigned long long>(__popc(ok_mask));
-    const double rank_dv = __longlong_as_double(static_cast<long long>(rank_bits));
-    if (lane < m) {
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(g.arcs + gbeg));
-    }
-    for (int p0 = 0; p0 < ptot; p0 += 32 * kUnroll) {
+    const int deg = ok ? entry.deg : 0;
+    const int most = __reduce_max_sync(kFullMask, deg);
+    const int with_arcs = __ffs(__ballot_sync(kFullMask, deg > 0)) - 1;
+    const uint32_t some_beg = __shfl_sync(kFullMask, entry.beg, with_arcs < 0 ? 0 : with_arcs);
+    const double dvs = __longlong_as_double(static_cast<long long>(v_bits));
+    const Arc* const arcs = sh.args.arcs + (deg > 0 ? entry.beg : some_beg);
+    for (int a0 = 0; a0 < most; a0 += kUnroll) {
         int x[kUnroll];
-        int src[kUnroll];
         double nd[kUnroll];
         unsigned long long cur[kUnroll];
         uint32_t eidx[kUnroll];
-        bool valid[kUnroll];
 #pragma unroll
         for (int u = 0; u < kUnroll; ++u) {
-            const int q = p0 + u * 32 + lane;
-            // the entry of pair q: the last one whose pairs start at or below q
-            int e = 0;
-#pragma unroll
-            for (int step = 16; step > 0; step >>= 1) {
-                const int c = e + step;
-                const int sc = __shfl_sync(kFullMask, si, c & 31);
-                e = (c < m && sc <= q) ? c : e;
-            }
-            const int local = q - __shfl_sync(kFullMask, si, e);
-            const int ke = __shfl_sync(kFullMask, ki, e);
-            const int a = (local * __shfl_sync(kFullMask, mgi, e)) >> 16;
-            const int t = (__shfl_sync(kFullMask, ri, e) + local - a * ke) & 31;
-            const int64_t beg_e = __shfl_sync(kFullMask, gbeg, e);
-            src[u] = __shfl_sync(kFullMask, rank_src, t);
-            const double dvs = __shfl_sync(kFullMask, rank_dv, t);
-            valid[u] = q < ptot && ((ok_mask >> t) & 1u);
-            eidx[u] = static_cast<uint32_t>(beg_e + a);
-            x[u] = 0;
-            nd[u] = 0.0;
-            cur[u] = 0ull;
-            if (valid[u]) {
-                const Arc arc = ldg_arc(&g.arcs[beg_e + a]);
-                x[u] = arc.col;
-                nd[u] = __dadd_rn(dvs, arc.len);
-                cur[u] = __ldcg(&dist[static_cast<int64_t>(x[u]) * kTile + src[u]]);
-            }
+            // a lane past its last arc reads its first one again (a lane without arcs: another lane's) and relaxes nothing
+            const int a = a0 + u;
+            const Arc arc = ldg_arc(&arcs[a < deg ? a : 0]);
+            x[u] = arc.col;
+            eidx[u] = entry.beg + static_cast<uint32_t>(a);
+            nd[u] = a < deg ? __dadd_rn(dvs, arc.len) : INFINITY;
+            cur[u] = __ldcg(&dist_s[static_cast<int64_t>(x[u]) * kTile]);
         }
-        relax_pairs<kUnroll, kTrack, kReach>(x, src, nd, cur, eidx, valid, dist, pend_nxt, far, theta, pred_key, tie, reach);
+        relax_lane<kUnroll, kTrack, kReach>(x, src, nd, cur, eidx, dist_s, sh);
     }
 }
 
@@ -431,18 +493,23 @@ __device__ __forceinline__ void packed_expand(const DeviceCsr& g, int m, int gv,
 // lane j fetches entry j's vertex, its pending mask, far marks and row offsets (one round of parallel loads), clears the
 // mask and the superseded far marks, and the warp then expands the vertices one after another: one at a time when a
 // vertex has a loop iteration's worth of (arc, source) pairs or more, else with its small neighbours in the chunk.
+// Not inlined: the registers of the other phases are saved around the call instead of being spilled inside its loops.
 template <int kUnroll, bool kTrack, bool kReach>
-__device__ __forceinline__ void expand_queue(const DeviceCsr& g, const int32_t* q_cur, int qlen, int lane, int* grab, int group_warps,
-                                             unsigned long long* __restrict__ dist, uint32_t* pend_cur, uint32_t* pend_nxt, uint32_t* far,
-                                             double theta, unsigned long long& expansions, unsigned long long& lane_expansions,
-                                             unsigned long long* pred_key, uint32_t* tie, unsigned long long* last, const Reach& reach) {
+__device__ __noinline__ void expand_queue() {
+    extern __shared__ __align__(16) unsigned long long smem[];
+    TileSmem& sh = *reinterpret_cast<TileSmem*>(smem);
+    const int lane = threadIdx.x & 31;
+    WarpScratch& w = sh.warp[threadIdx.x >> 5];
+    WarpWork& work = sh.work[threadIdx.x >> 5];
     for (;;) {
         int base = 0;
         int chunk = 0;
+        const int qlen = sh.ctl.qlen[sh.ctl.cur];
         if (lane == 0) {
             // the grab counter is in shared memory for single-CTA tiles and in global memory for groups: a volatile
             // generic load reads either (for global memory, from L2)
-            chunk = expand_chunk(qlen - *reinterpret_cast<volatile int*>(grab), group_warps);
+            int* const grab = sh.args.grab;
+            chunk = expand_chunk(qlen - *reinterpret_cast<volatile int*>(grab), sh.args.group_warps);
             base = atomicAdd(grab, chunk);
         }
         base = __shfl_sync(kFullMask, base, 0);
@@ -450,29 +517,32 @@ __device__ __forceinline__ void expand_queue(const DeviceCsr& g, const int32_t* 
         if (base >= qlen) {
             break;
         }
-        const int i = base + lane;
         const int count = qlen - base < chunk ? qlen - base : chunk;
-        int vj = 0;
-        uint32_t mj = 0;
-        int64_t bj = 0;
-        int dj = 0;
+        QueueEntry mine{ 0, 0u, 0u, 0 };
         if (lane < count) {
-            vj = __ldcg(&q_cur[i]);
-            mj = __ldcg(&pend_cur[vj]);
-            const uint32_t fm = __ldcg(&far[vj]);
-            bj = __ldg(&g.row_ptr[vj]);
-            dj = static_cast<int>(__ldg(&g.row_ptr[vj + 1]) - bj);
-            if (mj != 0u) {
-                pend_cur[vj] = 0u;
-                if (fm & mj) {
-                    atomicAnd(&far[vj], ~mj);  // those far marks are superseded by the near values expanded now
+            const uint32_t n_slot = sh.args.n_slot;
+            const int cur = sh.ctl.cur;
+            uint32_t* const pend_cur = sh.args.marks + static_cast<size_t>(cur) * n_slot;
+            uint32_t* const far = sh.args.marks + static_cast<size_t>(2) * n_slot;
+            mine.v = __ldcg(&sh.args.queue[static_cast<size_t>(cur) * n_slot + static_cast<uint32_t>(base + lane)]);
+            mine.mask = __ldcg(&pend_cur[mine.v]);
+            const uint32_t fm = __ldcg(&far[mine.v]);
+            const int64_t beg = __ldg(&sh.args.row_ptr[mine.v]);
+            mine.beg = static_cast<uint32_t>(beg);  // arc indices are 32-bit (predecessor keys, reverse CSR)
+            mine.deg = static_cast<int>(__ldg(&sh.args.row_ptr[mine.v + 1]) - beg);
+            if (mine.mask != 0u) {
+                pend_cur[mine.v] = 0u;
+                if (fm & mine.mask) {
+                    atomicAnd(&far[mine.v], ~mine.mask);  // those far marks are superseded by the near values expanded now
                 }
             }
         }
+        w.entry[lane] = mine;
+        __syncwarp();
         // entries with fewer pairs than one loop iteration holds go in groups (packed_expand), the others one by one
-        const int kj = __popc(mj);
-        const unsigned any_mask = __ballot_sync(kFullMask, lane < count && mj != 0u);
-        const unsigned small_mask = __ballot_sync(kFullMask, lane < count && mj != 0u && kj * dj < kPackPairs);
+        const int kj = __popc(mine.mask);
+        const unsigned any_mask = __ballot_sync(kFullMask, mine.mask != 0u);
+        const unsigned small_mask = __ballot_sync(kFullMask, mine.mask != 0u && kj * mine.deg < kPackPairs);
         int j = 0;
         while (j < count) {
             const unsigned rest = any_mask & ~((1u << j) - 1u);
@@ -480,14 +550,14 @@ __device__ __forceinline__ void expand_queue(const DeviceCsr& g, const int32_t* 
                 break;
             }
             j = __ffs(rest) - 1;  // the next entry with pending sources
-            unsigned fit = 0u;
             if ((small_mask >> j) & 1u) {
                 // the small entries from j up to the next large one, as many as hold 32 pending sources
                 const unsigned large_after = any_mask & ~small_mask & ~((1u << j) - 1u);
                 const int stop = large_after != 0u ? __ffs(large_after) - 1 : 32;
                 const unsigned run = small_mask & ~((1u << j) - 1u) & (stop >= 32 ? kFullMask : ((1u << stop) - 1u));
                 const bool in_run = (run >> lane) & 1u;
-                int kin = in_run ? kj : 0;
+                const int kl = in_run ? __popc(w.entry[lane].mask) : 0;
+                int kin = kl;
 #pragma unroll
                 for (int off = 1; off < 32; off <<= 1) {
                     const int ku = __shfl_up_sync(kFullMask, kin, off);
@@ -495,28 +565,32 @@ __device__ __forceinline__ void expand_queue(const DeviceCsr& g, const int32_t* 
                         kin += ku;
                     }
                 }
-                fit = __ballot_sync(kFullMask, in_run && kin <= 32);
-            }
-            if (__popc(fit) > 1) {
+                const bool in_fit = in_run && kin <= 32;
+                const unsigned fit = __ballot_sync(kFullMask, in_fit);
                 const int m = __popc(fit);
-                const int sl = lane < m ? static_cast<int>(__fns(fit, 0, lane + 1)) : 0;
-                const int gv = __shfl_sync(kFullMask, vj, sl);
-                const uint32_t gmask = __shfl_sync(kFullMask, mj, sl);
-                const int64_t gbeg = __shfl_sync(kFullMask, bj, sl);
-                const int gdeg = __shfl_sync(kFullMask, dj, sl);
-                packed_expand<kUnroll, kTrack, kReach>(g, m, gv, gmask, gbeg, gdeg, lane, dist, pend_nxt, far, theta, expansions,
-                                                       lane_expansions, pred_key, tie, last, reach);
-                j = 32 - __clz(fit);
-            } else {
-                const uint32_t amask = __shfl_sync(kFullMask, mj, j);
-                const int v = __shfl_sync(kFullMask, vj, j);
-                const int64_t beg = __shfl_sync(kFullMask, bj, j);
-                const int deg = __shfl_sync(kFullMask, dj, j);
-                batched_expand<kUnroll, kTrack, kReach>(g, v, amask, beg, deg, lane, dist, pend_nxt, far, theta, expansions, lane_expansions,
-                                                        pred_key, tie, last, reach);
-                ++j;
+                const int most = __reduce_max_sync(kFullMask, in_fit ? w.entry[lane].deg : 0);
+                // lane by lane the group takes `most` steps, kUnroll at a time; one by one, each entry takes a round of
+                // filter reads and one or two of distance reads
+                if (m > 1 && most <= 4 * m) {
+                    if (in_fit) {
+                        int at = kin - kl;
+                        for (uint32_t mask = w.entry[lane].mask; mask != 0u; mask &= mask - 1u) {
+                            w.rank[at++] = lane << 5 | (__ffs(mask) - 1);
+                        }
+                    }
+                    const int last_lane = 31 - __clz(fit);
+                    const int ktot = __shfl_sync(kFullMask, kin, last_lane);
+                    __syncwarp();
+                    packed_expand<kUnroll, kTrack, kReach>(sh, w, work, m, ktot, lane);
+                    __syncwarp();  // the next group overwrites rank
+                    j = last_lane + 1;
+                    continue;
+                }
             }
+            batched_expand<kUnroll, kTrack, kReach>(sh, w, work, j, lane);
+            ++j;
         }
+        __syncwarp();  // the next chunk overwrites the entries
     }
 }
 
@@ -547,18 +621,20 @@ __device__ __forceinline__ void compact_queue(const uint32_t* pend, int32_t* q, 
 // kMulti: the launch may put several CTAs on a tile (p.group_size > 1, cooperative launch); without it the group is
 // the CTA itself, whose control block lives in shared memory. kReach: the tiles keep reach lists.
 template <int kMode, int kUnroll, int kBlock, int kMinBlocks, bool kMulti = false, bool kReach = false>
-__global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const SsspParams p, const BrandesParams b) {
+__global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_constant__ SsspParams p, const __grid_constant__ BrandesParams b) {
     extern __shared__ __align__(16) unsigned long long smem[];
     unsigned long long* s_acc_sum = smem;                                // kTile * kAccDigits
     unsigned long long* s_acc_inv = smem + kTile * kAccDigits;          // kTile * kAccDigits
-    unsigned int* s_hist = reinterpret_cast<unsigned int*>(smem + 2 * kTile * kAccDigits);
-    __shared__ TileShared s;
+    static_assert(kBlock <= 32 * kMaxWarps, "one warp scratch per warp");
+    TileSmem& sh = *reinterpret_cast<TileSmem*>(smem);
+    unsigned int* s_hist = reinterpret_cast<unsigned int*>(&sh + 1);
+    unsigned long long* s_part = smem + 2 * kTile * kAccDigits;  // kBlock + 3 words
+    TileShared& s = sh.ctl;
     __shared__ unsigned s_bar;
     __shared__ int s_src[kTile];
     __shared__ unsigned long long s_unreach[kTile];
     __shared__ unsigned long long s_arcs[kTile];
     __shared__ unsigned long long s_max[kTile];
-    __shared__ unsigned long long s_part[kBlock + 3];
 
     const int tid = threadIdx.x;
     const int lane = tid & 31;
@@ -590,15 +666,18 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const SsspPara
 #define NGX_GW (kMulti ? static_cast<int>(blockIdx.x % p.group_size) * static_cast<int>(blockDim.x >> 5) + static_cast<int>(threadIdx.x >> 5) \
                        : static_cast<int>(threadIdx.x >> 5))
 #define NGX_GWARPS (kMulti ? p.group_size * static_cast<int>(blockDim.x >> 5) : static_cast<int>(blockDim.x >> 5))
-    unsigned long long expansions = 0, lane_expansions = 0;
+    if (lane == 0) {
+        sh.work[warp] = WarpWork{ 0ull, 0ull };
+    }
 
     unsigned long long* dist = p.ws_dist + slot * n_slot * kTile;
-    uint32_t* pend0 = p.ws_pend + slot * 2 * n_slot;
+    uint32_t* pend0 = p.ws_pend + slot * 3 * n_slot;
     uint32_t* pend1 = pend0 + n_slot;
-    uint32_t* far = p.ws_far + slot * n_slot;
+    uint32_t* far = pend1 + n_slot;
     int32_t* q0 = p.ws_queue + slot * 2 * n_slot;
     int32_t* q1 = q0 + n_slot;
     uint32_t* stamp = p.ws_stamp + slot * n_slot;
+    uint8_t* const bound = reinterpret_cast<uint8_t*>(stamp);
     // reach lists: compiled in only for the kernels that keep them (kReach), so the others carry no extra registers
     const Reach reach{ kReach ? p.ws_reach + slot * n_slot : nullptr, kReach ? p.ws_touched + slot * n_slot : nullptr,
                        kReach ? &ctl()->touched_len : nullptr };
@@ -648,13 +727,10 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const SsspPara
         pend0[i] = 0u;
         pend1[i] = 0u;
         far[i] = 0u;
-        stamp[i] = 0u;
+        bound[i] = kNoBound;
         if (kReach) {
             reach.mask[i] = 0u;
         }
-    }
-    for (int i = tid; i < 2 * kTile * kAccDigits; i += blockDim.x) {
-        smem[i] = 0ull;
     }
     for (int i = tid; i < p.out.hist_bins; i += blockDim.x) {
         s_hist[i] = 0u;
@@ -711,6 +787,11 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const SsspPara
             s_arcs[tid] = 0ull;
             s_max[tid] = 0ull;
         }
+        if (tid == 0) {
+            sh.args = ExpandArgs{ g.arcs, g.row_ptr, dist, pend0, q0, bound, &ctl()->grab, reinterpret_cast<unsigned long long*>(sigma),
+                                  reinterpret_cast<unsigned long long*>(delta), tie, reach, static_cast<uint32_t>(n_slot), nsrc,
+                                  static_cast<int>(static_cast<uint32_t>(__double2hiint(0.25 * gd.delta)) >> 15), NGX_GWARPS };
+        }
         __syncthreads();
         if ((!kMulti || grp().rank == 0) && warp == 0) {
             const int v = s_src[lane];
@@ -736,14 +817,9 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const SsspPara
                 if (qlen == 0) {
                     break;
                 }
-                uint32_t* pend_cur = cur ? pend1 : pend0;
                 uint32_t* pend_nxt = cur ? pend0 : pend1;
-                const int32_t* q_cur = cur ? q1 : q0;
                 int32_t* q_nxt = cur ? q0 : q1;
-                const double theta = s.theta;
-                expand_queue<kUnroll, kMode != kModeApsp, kReach>(g, q_cur, qlen, lane, &ctl()->grab, NGX_GWARPS, dist, pend_cur, pend_nxt,
-                                                          far, theta, expansions, lane_expansions, reinterpret_cast<unsigned long long*>(sigma), tie,
-                                                          reinterpret_cast<unsigned long long*>(delta), reach);
+                expand_queue<kUnroll, kMode != kModeApsp, kReach>();
                 sync([&](volatile TileShared& c) {
                     c.qlen[cur] = 0;
                     c.grab = 0;
@@ -841,6 +917,12 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const SsspPara
         if (s.stop != 0) {
             break;
         }
+        // the expansions borrowed the epilogue's accumulators, which must start at zero (the barrier that ended the
+        // distance phase separates the two)
+        for (int i = tid; i < 2 * kTile * kAccDigits; i += blockDim.x) {
+            smem[i] = 0ull;
+        }
+        __syncthreads();
 
         if (tid == 0) {
             const long long now = clock64();
@@ -864,6 +946,11 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const SsspPara
                 dag_fill<kMode == kModeBrandes>(rg, b.arc_src, n, dist, cnt, pred, soff, scnt, succ, lane, NGX_GW, NGX_GWARPS);
                 sync0();
                 dag_sort(soff, succ, nt, NGX_GT, NGX_GTHREADS);
+            }
+            if (!use_lists) {
+                for (int64_t i = NGX_GT; i < n; i += NGX_GTHREADS) {
+                    stamp[i] = 0u;  // its words held the distance phase's bounds until here
+                }
             }
             sync([&](volatile TileShared& c) {
                 if (!use_lists) {
@@ -1031,8 +1118,15 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const SsspPara
         }
         for (int64_t i = NGX_GW; i < span; i += NGX_GWARPS) {
             const int64_t v = by_list ? static_cast<int64_t>(__ldcg(&reach.list[i])) : i;
-            if (kReach && lane == 0) {
-                reach.mask[v] = 0u;
+            if (lane == 0) {
+                if constexpr (kMode == kModeApsp) {
+                    bound[v] = kNoBound;
+                } else {
+                    stamp[v] = 0xFFFFFFFFu;  // whole words: stamps reach past the graph's n bounds, into a larger graph's
+                }
+                if (kReach) {
+                    reach.mask[v] = 0u;
+                }
             }
             unsigned long long* slot_ptr = &dist[v * kTile + lane];
             const unsigned long long bits = __ldcg(slot_ptr);
@@ -1172,18 +1266,14 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const SsspPara
             }
         }
         __syncthreads();
-        for (int i = tid; i < 2 * kTile * kAccDigits; i += blockDim.x) {
-            smem[i] = 0ull;
-        }
-        __syncthreads();
         if (tid == 0) {
             atomicAdd(&cnts[kCyclesEpilogue], static_cast<unsigned long long>(clock64() - t_phase));
         }
     }
-    if (lane == 0 && expansions != 0) {
+    if (lane == 0 && sh.work[warp].expansions != 0) {
         // whole-launch totals, kept in the first graph's counters
-        atomicAdd(&p.out.counters[kExpansions], expansions);
-        atomicAdd(&p.out.counters[kLaneExpansions], lane_expansions);
+        atomicAdd(&p.out.counters[kExpansions], sh.work[warp].expansions);
+        atomicAdd(&p.out.counters[kLaneExpansions], sh.work[warp].lane_expansions);
     }
 #undef NGX_GT
 #undef NGX_GTHREADS
@@ -1358,9 +1448,9 @@ __global__ void __launch_bounds__(512, 2) sssp_plain_kernel(const SsspParams p, 
     unsigned long long expansions = 0;
 
     unsigned long long* dist = p.ws_dist + slot * n;
-    uint32_t* pend0 = p.ws_pend + slot * 2 * n;
+    uint32_t* pend0 = p.ws_pend + slot * 3 * n;
     uint32_t* pend1 = pend0 + n;
-    uint32_t* far = p.ws_far + slot * n;
+    uint32_t* far = pend1 + n;
     int32_t* q0 = p.ws_queue + slot * 2 * n;
     int32_t* q1 = q0 + n;
     uint32_t* stamp = p.ws_stamp + slot * n;
