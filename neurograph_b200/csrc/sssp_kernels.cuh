@@ -206,19 +206,19 @@ constexpr int kAccBytes = 2 * kTile * kAccDigits * 8;
 struct ExpandArgs {
     const Arc* arcs;
     const int64_t* row_ptr;
+    const Arc* rarcs;             // in-arcs (DAG passes)
+    const int64_t* rrow_ptr;
     unsigned long long* dist;
     uint32_t* marks;              // pending masks of even and odd iterations, far marks: three times n_slot words
     int32_t* queue;               // two queues of n_slot entries
     uint8_t* bound;
     int* grab;
-    unsigned long long* pred_key;
-    unsigned long long* last;
-    uint32_t* tie;
     Reach reach;
     uint32_t n_slot;
     int nsrc;
     int bound_base;
     int group_warps;
+    int n;
 };
 
 // Dynamic shared memory of the tile kernel, before the histogram. The distance phase's warp scratch overlays the
@@ -234,46 +234,28 @@ static_assert(sizeof(WarpScratch) * kMaxWarps >= kAccBytes + (512 + 3) * 8, "acc
 static_assert(sizeof(TileSmem) % 16 == 0, "the histogram follows");
 
 // The relaxations of kUnroll arcs by this lane's source, their loads done: arc u relaxes d[x[u]][src] with nd[u] (cur[u] =
-// the distance read before); an infinite nd[u] relaxes nothing. The atomic minima are issued back to back and waited for
-// together (APSP mode: not waited for at all), then the marks; see batched_expand for what each mode does with an
-// improvement. dist_s points at the source's column.
-template <int kUnroll, bool kTrack, bool kReach>
-__device__ __forceinline__ void relax_lane(const int (&x)[kUnroll], int src, const double (&nd)[kUnroll], unsigned long long (&cur)[kUnroll],
-                                           const uint32_t (&eidx)[kUnroll], unsigned long long* dist_s, const TileSmem& sh) {
-    bool tried[kUnroll];
+// the distance read before); an infinite nd[u] relaxes nothing. The atomic minima are issued back to back and not waited
+// for, then the marks. dist_s points at the source's column. With reach lists (kReach) the old value is needed: the first
+// finite distance of (x, s) appends x to the tile's reached vertices.
+template <int kUnroll, bool kReach>
+__device__ __forceinline__ void relax_lane(const int (&x)[kUnroll], int src, const double (&nd)[kUnroll], const unsigned long long (&cur)[kUnroll],
+                                           unsigned long long* dist_s, const TileSmem& sh) {
 #pragma unroll
     for (int u = 0; u < kUnroll; ++u) {
         const unsigned long long nb = static_cast<unsigned long long>(__double_as_longlong(nd[u]));
-        tried[u] = nb < cur[u] || (kTrack && nb == cur[u] && nb != kInfBits);
-        if (tried[u]) {
-            if constexpr (kTrack) {
-                // an equal value is a tie already (the minimum would return it unchanged)
-                cur[u] = nb < cur[u] ? atomicMin(&dist_s[static_cast<int64_t>(x[u]) * kTile], nb) : nb;
-            } else {
-                atomicMin(&dist_s[static_cast<int64_t>(x[u]) * kTile], nb);
-            }
+        if (nb < cur[u]) {
+            atomicMin(&dist_s[static_cast<int64_t>(x[u]) * kTile], nb);
         }
     }
     const uint32_t bit = 1u << src;
 #pragma unroll
     for (int u = 0; u < kUnroll; ++u) {
-        if (tried[u]) {
-            const unsigned long long nb = static_cast<unsigned long long>(__double_as_longlong(nd[u]));
-            const unsigned long long old = cur[u];
-            if constexpr (kTrack) {
-                if (nb < old) {
-                    atomicMin(&sh.args.pred_key[static_cast<int64_t>(x[u]) * kTile + src], ((nb >> 32) << 32) | eidx[u]);
-                } else if (nb == old) {
-                    atomicOr(&sh.args.tie[x[u]], bit);
-                }
+        if (static_cast<unsigned long long>(__double_as_longlong(nd[u])) < cur[u]) {
+            if (kReach && cur[u] == kInfBits) {
+                sh.args.reach.add(x[u], bit);
             }
-            if (!kTrack || nb < old) {
-                if (kReach && old == kInfBits) {
-                    sh.args.reach.add(x[u], bit);  // the first distance of (x, s): x joins the tile's reached vertices
-                }
-                const uint32_t which = nd[u] < sh.ctl.theta ? static_cast<uint32_t>(sh.ctl.cur ^ 1) : 2u;
-                atomicOr(&sh.args.marks[static_cast<size_t>(which) * sh.args.n_slot + static_cast<uint32_t>(x[u])], bit);
-            }
+            const uint32_t which = nd[u] < sh.ctl.theta ? static_cast<uint32_t>(sh.ctl.cur ^ 1) : 2u;
+            atomicOr(&sh.args.marks[static_cast<size_t>(which) * sh.args.n_slot + static_cast<uint32_t>(x[u])], bit);
         }
     }
 }
@@ -317,45 +299,26 @@ constexpr int kFilterDegree = 16;
 // An improvement below theta sets the pair's bit in pend_nxt (the next iteration's queue is compacted from those
 // masks after the iteration), one at or above theta its far mark. The kUnroll relaxations of a lane are issued back
 // to back and waited for together.
-// APSP mode: the atomic minimum is not waited for. An improvement is judged against the distance read before it, so
+// The atomic minimum is not waited for. An improvement is judged against the distance read before it, so
 // a relaxation that lost a race to a smaller value may still set a pending bit or a far mark: the pair is then
 // expanded once more with its (smaller) current distance, or its superseded far mark is cleared or moved by the next
 // expansion or bucket step, which changes the work and never the fixed point.
-// kTrack (betweenness / adjoint): the atomic minimum returns the old value. Each improvement of d[x][s] to nb offers
-// the key (top 32 bits of nb, arc index) to pred_key[x][s] with an atomic minimum, so the key of the smallest
-// distance wins whatever the order of the stores; a relaxation that ties with d[x][s] sets bit s of tie[x]. Every
-// DAG arc is relaxed with final distances, so a (x, s) whose tie bit stayed clear has exactly one DAG predecessor: the
-// arc in its key (the DAG count pass checks it). For that, no (v, s) may be expanded twice with one distance (the
-// repeat would look like a tie): last[v][s] keeps the distance of the latest expansion, and sources whose distance has
-// not changed since are dropped from the next.
 // The caller has taken v's pending mask (entry.mask, non-zero) and cleared it and v's superseded far marks: see
 // expand_queue. Lanes >= nsrc hold no source.
-template <int kUnroll, bool kTrack, bool kReach>
+template <int kUnroll, bool kReach>
 __device__ __forceinline__ void batched_expand(TileSmem& sh, WarpScratch& w, WarpWork& work, int j, int lane) {
     const QueueEntry entry = w.entry[j];
-    uint32_t amask = entry.mask;
+    const uint32_t amask = entry.mask;
     unsigned long long* const dist = sh.args.dist;
     const Arc* const arcs = sh.args.arcs + entry.beg;
     const int64_t vrow = static_cast<int64_t>(entry.v) * kTile + lane;
     const unsigned long long row_bits = __ldcg(&dist[vrow]);
     const uint32_t row_hi = static_cast<uint32_t>(row_bits >> 32);
-    if constexpr (kTrack) {
-        unsigned long long* const last = sh.args.last;
-        const bool pending = (amask >> lane) & 1u;
-        const bool repeat = pending && __ldcg(&last[vrow]) == row_bits;
-        if (pending && !repeat) {
-            last[vrow] = row_bits;
-        }
-        amask &= ~__ballot_sync(kFullMask, repeat);
-    }
     const int bound_base = sh.args.bound_base;
     const uint32_t row_max = __reduce_max_sync(kFullMask, lane < sh.args.nsrc ? row_hi : 0u);
     const int max_key = bound_key(row_max, bound_base);
     if (lane == 0 && max_key < kNoBound) {
         sh.args.bound[entry.v] = static_cast<uint8_t>(max_key > 0 ? max_key : 0);
-    }
-    if (amask == 0u) {
-        return;
     }
     const uint32_t min_hi = __reduce_min_sync(kFullMask, ((amask >> lane) & 1u) != 0u ? row_hi : 0xFFFFFFFFu);
     const double d_min = __hiloint2double(static_cast<int>(min_hi), 0);  // at most every pending distance
@@ -412,18 +375,16 @@ __device__ __forceinline__ void batched_expand(TileSmem& sh, WarpScratch& w, War
             int x[kUnroll];
             double nd[kUnroll];
             unsigned long long cur[kUnroll];
-            uint32_t eidx[kUnroll];
 #pragma unroll
             for (int u = 0; u < kUnroll; ++u) {
                 // a lane without a pair reads the first kept arc's and relaxes nothing
                 const Arc kept_arc = w.kept[a < kept ? a : 0];
                 x[u] = kept_arc.col;
-                eidx[u] = entry.beg + static_cast<uint32_t>(kept_arc.id);
                 nd[u] = a < kept ? __dadd_rn(dvs, kept_arc.len) : INFINITY;
                 cur[u] = __ldcg(&dist_s[static_cast<int64_t>(x[u]) * kTile]);
                 a += step_a;
             }
-            relax_lane<kUnroll, kTrack, kReach>(x, src, nd, cur, eidx, dist_s, sh);
+            relax_lane<kUnroll, kReach>(x, src, nd, cur, dist_s, sh);
         }
         __syncwarp();  // the next block of arcs (the next vertex) overwrites kept (and rank)
     }
@@ -439,32 +400,20 @@ constexpr int kPackPairs = NGX_PACK_PAIRS;
 // Expands a group of m small queue entries together: w.rank[t], t < ktot <= 32, names the t-th (entry, pending source) of
 // the group. Lane t takes it and walks its entry's arcs, kUnroll at a time: the lanes of an entry read the same arc
 // records and neighbouring distances of the same rows, no lane needs to find its pairs, and the group takes as long as
-// its entry with the most arcs. The relaxations, the repeat check of the DAG modes and the counters are
-// batched_expand's; the arcs are not filtered (a bound read per arc would cost as much as the few distance reads it
+// its entry with the most arcs. The relaxations and the counters are batched_expand's; the arcs are not filtered (a bound read per arc would cost as much as the few distance reads it
 // saves).
-template <int kUnroll, bool kTrack, bool kReach>
+template <int kUnroll, bool kReach>
 __device__ __forceinline__ void packed_expand(TileSmem& sh, WarpScratch& w, WarpWork& work, int m, int ktot, int lane) {
     const int code = w.rank[lane < ktot ? lane : 0];
     const int src = code & 31;
     const QueueEntry entry = w.entry[code >> 5];
-    const int64_t vrow = static_cast<int64_t>(entry.v) * kTile + src;
     unsigned long long* const dist_s = sh.args.dist + src;
     const unsigned long long v_bits = __ldcg(&dist_s[static_cast<int64_t>(entry.v) * kTile]);
-    bool ok = lane < ktot;
-    if constexpr (kTrack) {
-        unsigned long long* const last = sh.args.last;
-        if (ok && __ldcg(&last[vrow]) == v_bits) {
-            ok = false;  // expanded with this distance already
-        } else if (ok) {
-            last[vrow] = v_bits;
-        }
-    }
-    const unsigned ok_mask = __ballot_sync(kFullMask, ok);
-    if (lane == 0 && ok_mask != 0u) {
+    if (lane == 0) {
         work.expansions += static_cast<unsigned long long>(m);
-        work.lane_expansions += static_cast<unsigned long long>(__popc(ok_mask));
+        work.lane_expansions += static_cast<unsigned long long>(ktot);
     }
-    const int deg = ok ? entry.deg : 0;
+    const int deg = lane < ktot ? entry.deg : 0;
     const int most = __reduce_max_sync(kFullMask, deg);
     const int with_arcs = __ffs(__ballot_sync(kFullMask, deg > 0)) - 1;
     const uint32_t some_beg = __shfl_sync(kFullMask, entry.beg, with_arcs < 0 ? 0 : with_arcs);
@@ -474,18 +423,16 @@ __device__ __forceinline__ void packed_expand(TileSmem& sh, WarpScratch& w, Warp
         int x[kUnroll];
         double nd[kUnroll];
         unsigned long long cur[kUnroll];
-        uint32_t eidx[kUnroll];
 #pragma unroll
         for (int u = 0; u < kUnroll; ++u) {
             // a lane past its last arc reads its first one again (a lane without arcs: another lane's) and relaxes nothing
             const int a = a0 + u;
             const Arc arc = ldg_arc(&arcs[a < deg ? a : 0]);
             x[u] = arc.col;
-            eidx[u] = entry.beg + static_cast<uint32_t>(a);
             nd[u] = a < deg ? __dadd_rn(dvs, arc.len) : INFINITY;
             cur[u] = __ldcg(&dist_s[static_cast<int64_t>(x[u]) * kTile]);
         }
-        relax_lane<kUnroll, kTrack, kReach>(x, src, nd, cur, eidx, dist_s, sh);
+        relax_lane<kUnroll, kReach>(x, src, nd, cur, dist_s, sh);
     }
 }
 
@@ -494,7 +441,7 @@ __device__ __forceinline__ void packed_expand(TileSmem& sh, WarpScratch& w, Warp
 // mask and the superseded far marks, and the warp then expands the vertices one after another: one at a time when a
 // vertex has a loop iteration's worth of (arc, source) pairs or more, else with its small neighbours in the chunk.
 // Not inlined: the registers of the other phases are saved around the call instead of being spilled inside its loops.
-template <int kUnroll, bool kTrack, bool kReach>
+template <int kUnroll, bool kReach>
 __device__ __noinline__ void expand_queue() {
     extern __shared__ __align__(16) unsigned long long smem[];
     TileSmem& sh = *reinterpret_cast<TileSmem*>(smem);
@@ -528,7 +475,7 @@ __device__ __noinline__ void expand_queue() {
             mine.mask = __ldcg(&pend_cur[mine.v]);
             const uint32_t fm = __ldcg(&far[mine.v]);
             const int64_t beg = __ldg(&sh.args.row_ptr[mine.v]);
-            mine.beg = static_cast<uint32_t>(beg);  // arc indices are 32-bit (predecessor keys, reverse CSR)
+            mine.beg = static_cast<uint32_t>(beg);  // arc indices are 32-bit, as in the reverse CSR
             mine.deg = static_cast<int>(__ldg(&sh.args.row_ptr[mine.v + 1]) - beg);
             if (mine.mask != 0u) {
                 pend_cur[mine.v] = 0u;
@@ -581,16 +528,182 @@ __device__ __noinline__ void expand_queue() {
                     const int last_lane = 31 - __clz(fit);
                     const int ktot = __shfl_sync(kFullMask, kin, last_lane);
                     __syncwarp();
-                    packed_expand<kUnroll, kTrack, kReach>(sh, w, work, m, ktot, lane);
+                    packed_expand<kUnroll, kReach>(sh, w, work, m, ktot, lane);
                     __syncwarp();  // the next group overwrites rank
                     j = last_lane + 1;
                     continue;
                 }
             }
-            batched_expand<kUnroll, kTrack, kReach>(sh, w, work, j, lane);
+            batched_expand<kUnroll, kReach>(sh, w, work, j, lane);
             ++j;
         }
         __syncwarp();  // the next chunk overwrites the entries
+    }
+}
+
+// ------------------------------------------------------------------------------------------ shortest-path DAG
+// low[v] = high word of the smallest d[v][s] of the tile (final distances): a lower bound of every one of them.
+__device__ __forceinline__ void dag_low(const unsigned long long* dist, uint32_t* low, int64_t n, int nsrc, int lane, int gw, int gwarps) {
+    constexpr int kRows = 4;
+    for (int64_t v0 = gw; v0 < n; v0 += static_cast<int64_t>(kRows) * gwarps) {
+        uint32_t hi[kRows];
+#pragma unroll
+        for (int i = 0; i < kRows; ++i) {
+            const int64_t v = v0 + static_cast<int64_t>(i) * gwarps;
+            hi[i] = v < n && lane < nsrc ? static_cast<uint32_t>(__ldcg(&dist[v * kTile + lane]) >> 32) : 0xFFFFFFFFu;
+        }
+#pragma unroll
+        for (int i = 0; i < kRows; ++i) {
+            const int64_t v = v0 + static_cast<int64_t>(i) * gwarps;
+            const uint32_t least = __reduce_min_sync(kFullMask, hi[i]);
+            if (v < n && lane == 0) {
+                low[v] = least;
+            }
+        }
+    }
+}
+
+// Calls visit(u, e) in every lane in `active` for each DAG in-arc u -> v of its source (fl(d[u][s] + len) == d[v][s], e =
+// the arc's forward index), in reverse-CSR order. An arc can be on some source's DAG only if fl(low[u] + len) is at most
+// the largest d[v][s] (fl is monotone), so 128 in-arcs at a time are filtered with one 4-byte read each, and only the
+// rows of the rest (16 % at out-degree 100, 30-50 % at 40) are read, four rows in flight.
+template <typename Visit>
+__device__ __forceinline__ void scan_in_arcs(const TileSmem& sh, WarpScratch& w, const uint32_t* low, int v, unsigned long long dv, bool active,
+                                             int lane, const Visit& visit) {
+    const uint32_t dv_max = __reduce_max_sync(kFullMask, active ? static_cast<uint32_t>(dv >> 32) : 0u);
+    const int64_t beg = __ldg(&sh.args.rrow_ptr[v]);
+    const int deg = static_cast<int>(__ldg(&sh.args.rrow_ptr[v + 1]) - beg);
+    const Arc* const arcs = sh.args.rarcs + beg;
+    const unsigned long long* const dist_s = sh.args.dist + lane;
+    for (int a0 = 0; a0 < deg; a0 += kArcBlock) {
+        int kept = 0;
+        {
+            Arc arc[kArcBlock / 32];
+            uint32_t lo[kArcBlock / 32];
+#pragma unroll
+            for (int u = 0; u < kArcBlock / 32; ++u) {
+                const int i = a0 + u * 32 + lane;
+                arc[u] = ldg_arc_once(&arcs[i < deg ? i : deg - 1]);
+            }
+#pragma unroll
+            for (int u = 0; u < kArcBlock / 32; ++u) {
+                lo[u] = __ldcg(&low[arc[u].col]);
+            }
+#pragma unroll
+            for (int u = 0; u < kArcBlock / 32; ++u) {
+                const int i = a0 + u * 32 + lane;
+                const double least = __dadd_rn(__hiloint2double(static_cast<int>(lo[u]), 0), arc[u].len);
+                const bool keep = i < deg && static_cast<uint32_t>(__double2hiint(least)) <= dv_max;
+                const unsigned bal = __ballot_sync(kFullMask, keep);
+                if (keep) {
+                    w.kept[kept + __popc(bal & lanemask_lt())] = arc[u];
+                }
+                kept += __popc(bal);
+            }
+        }
+        __syncwarp();
+        constexpr int kRows = 4;
+        for (int a = 0; a < kept; a += kRows) {
+            unsigned long long du[kRows];
+#pragma unroll
+            for (int u = 0; u < kRows; ++u) {
+                du[u] = __ldcg(&dist_s[static_cast<int64_t>(w.kept[a + u < kept ? a + u : a].col) * kTile]);
+            }
+#pragma unroll
+            for (int u = 0; u < kRows; ++u) {
+                const Arc arc = w.kept[a + u < kept ? a + u : a];
+                if (a + u < kept && active && du[u] != kInfBits && on_dag(du[u], arc.len, dv)) {
+                    visit(arc.col, static_cast<uint32_t>(arc.id));
+                }
+            }
+        }
+        __syncwarp();  // the next block of arcs overwrites kept
+    }
+}
+
+// cnt[v][s] = DAG predecessors of (v, s), pred[v][s] = forward index of one of their arcs (the only one when cnt is 1),
+// scnt[u][s] += 1 for each DAG arc u -> v, sigma = 0; warp per vertex, lane per source. src_lane: this lane's source
+// vertex (-1 without one).
+__device__ __noinline__ void dag_count(const uint32_t* low, int src_lane, double* sigma, uint32_t* cnt, uint32_t* scnt, uint32_t* pred,
+                                       unsigned long long* active_pairs, int gw) {
+    extern __shared__ __align__(16) unsigned long long smem[];
+    TileSmem& sh = *reinterpret_cast<TileSmem*>(smem);
+    const int lane = threadIdx.x & 31;
+    WarpScratch& w = sh.warp[threadIdx.x >> 5];
+    unsigned active_count = 0;
+    for (int v = gw; v < sh.args.n; v += sh.args.group_warps) {
+        const int64_t row = static_cast<int64_t>(v) * kTile + lane;
+        const unsigned long long dv = __ldcg(&sh.args.dist[row]);
+        const bool active = src_lane >= 0 && dv != kInfBits && v != src_lane;
+        uint32_t c = 0;
+        uint32_t first = 0;
+        if (__ballot_sync(kFullMask, active) != 0u) {
+            active_count += active ? 1u : 0u;
+            scan_in_arcs(sh, w, low, v, dv, active, lane, [&](int u, uint32_t e) {
+                first = c == 0 ? e : first;
+                ++c;
+                atomicAdd(&scnt[static_cast<int64_t>(u) * kTile + lane], 1u);
+            });
+        }
+        sigma[row] = 0.0;
+        cnt[row] = c;
+        pred[row] = first;
+    }
+    const unsigned total = __reduce_add_sync(kFullMask, active_count);
+    if (lane == 0 && total != 0u) {
+        atomicAdd(active_pairs, static_cast<unsigned long long>(total));
+    }
+}
+
+// Fills the successor lists: each DAG arc u -> v is appended to (u, s), as its target v (kTarget: betweenness needs
+// nothing else) or as its forward-CSR index (the adjoint also needs the arc). A (v, s) with a single DAG predecessor
+// takes it from pred[v][s]; only vertices with several for some source scan their in-arcs again.
+template <bool kTarget>
+__device__ __noinline__ void dag_fill(const int32_t* arc_src, const uint32_t* low, const uint32_t* cnt, const uint32_t* pred, const uint32_t* soff,
+                                      uint32_t* sfill, uint32_t* succ, int gw) {
+    extern __shared__ __align__(16) unsigned long long smem[];
+    TileSmem& sh = *reinterpret_cast<TileSmem*>(smem);
+    const int lane = threadIdx.x & 31;
+    WarpScratch& w = sh.warp[threadIdx.x >> 5];
+    constexpr int kRows = 2;  // single-predecessor lanes of two vertices, their reads side by side
+    for (int v0 = gw; v0 < sh.args.n; v0 += kRows * sh.args.group_warps) {
+        uint32_t c[kRows], e[kRows], pos[kRows], off[kRows];
+        int64_t urow[kRows];
+#pragma unroll
+        for (int i = 0; i < kRows; ++i) {
+            const int64_t v = v0 + static_cast<int64_t>(i) * sh.args.group_warps;
+            c[i] = v < sh.args.n ? __ldcg(&cnt[v * kTile + lane]) : 0u;
+            e[i] = c[i] == 1u ? __ldcg(&pred[v * kTile + lane]) : 0u;
+        }
+#pragma unroll
+        for (int i = 0; i < kRows; ++i) {
+            urow[i] = c[i] == 1u ? static_cast<int64_t>(__ldg(&arc_src[e[i]])) * kTile + lane : 0;
+        }
+#pragma unroll
+        for (int i = 0; i < kRows; ++i) {
+            pos[i] = c[i] == 1u ? atomicAdd(&sfill[urow[i]], 1u) : 0u;
+            off[i] = c[i] == 1u ? __ldcg(&soff[urow[i]]) : 0u;
+        }
+#pragma unroll
+        for (int i = 0; i < kRows; ++i) {
+            if (c[i] == 1u) {
+                const int64_t v = v0 + static_cast<int64_t>(i) * sh.args.group_warps;
+                succ[off[i] + pos[i]] = kTarget ? static_cast<uint32_t>(v) : e[i];
+            }
+        }
+#pragma unroll 1
+        for (int i = 0; i < kRows; ++i) {
+            const int v = v0 + i * sh.args.group_warps;
+            const bool active = c[i] >= 2u;
+            if (v < sh.args.n && __ballot_sync(kFullMask, active) != 0u) {
+                const unsigned long long dv = __ldcg(&sh.args.dist[static_cast<int64_t>(v) * kTile + lane]);
+                scan_in_arcs(sh, w, low, v, dv, active, lane, [&](int u, uint32_t fwd) {
+                    const int64_t to = static_cast<int64_t>(u) * kTile + lane;
+                    const uint32_t at = atomicAdd(&sfill[to], 1u);
+                    succ[__ldcg(&soff[to]) + at] = kTarget ? static_cast<uint32_t>(v) : fwd;
+                });
+            }
+        }
     }
 }
 
@@ -692,7 +805,6 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
     uint32_t* scnt = nullptr;
     uint32_t* soff = nullptr;
     uint32_t* succ = nullptr;
-    uint32_t* tie = nullptr;
     if constexpr (kMode != kModeApsp) {
         scnt = b.ws_scnt + slot * nt_slot;
         soff = b.ws_soff + slot * (nt_slot + 1);
@@ -704,19 +816,8 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
         lvl = b.ws_lvl + slot * nt_slot;
         list = b.ws_list + slot * nt_slot;
         loff = b.ws_loff + slot * (n_slot + 2);
-        tie = b.ws_tie + slot * n_slot;
-        for (int64_t i = NGX_GT; i < n_slot; i += NGX_GTHREADS) {
-            tie[i] = 0u;
-        }
         for (int64_t i = NGX_GT; i < nt_slot; i += NGX_GTHREADS) {
             scnt[i] = 0u;
-            sigma[i] = __longlong_as_double(-1ll);  // all-ones: the empty predecessor key (sigma is zeroed by the count pass)
-            delta[i] = __longlong_as_double(-1ll);  // all-ones: no expansion yet (delta holds last[][] in the SSSP phase)
-            if constexpr (kMode == kModeGrad) {
-                delta_g[i] = 0.0;
-            }
-            cnt[i] = 0u;
-            lvl[i] = kNoLevel;
         }
     }
 
@@ -788,9 +889,9 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
             s_max[tid] = 0ull;
         }
         if (tid == 0) {
-            sh.args = ExpandArgs{ g.arcs, g.row_ptr, dist, pend0, q0, bound, &ctl()->grab, reinterpret_cast<unsigned long long*>(sigma),
-                                  reinterpret_cast<unsigned long long*>(delta), tie, reach, static_cast<uint32_t>(n_slot), nsrc,
-                                  static_cast<int>(static_cast<uint32_t>(__double2hiint(0.25 * gd.delta)) >> 15), NGX_GWARPS };
+            sh.args = ExpandArgs{ g.arcs, g.row_ptr, rg.arcs, rg.row_ptr, dist, pend0, q0, bound, &ctl()->grab, reach,
+                                  static_cast<uint32_t>(n_slot), nsrc, static_cast<int>(static_cast<uint32_t>(__double2hiint(0.25 * gd.delta)) >> 15),
+                                  NGX_GWARPS, static_cast<int>(n) };
         }
         __syncthreads();
         if ((!kMulti || grp().rank == 0) && warp == 0) {
@@ -819,7 +920,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
                 }
                 uint32_t* pend_nxt = cur ? pend0 : pend1;
                 int32_t* q_nxt = cur ? q0 : q1;
-                expand_queue<kUnroll, kMode != kModeApsp, kReach>();
+                expand_queue<kUnroll, kReach>();
                 sync([&](volatile TileShared& c) {
                     c.qlen[cur] = 0;
                     c.grab = 0;
@@ -917,13 +1018,6 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
         if (s.stop != 0) {
             break;
         }
-        // the expansions borrowed the epilogue's accumulators, which must start at zero (the barrier that ended the
-        // distance phase separates the two)
-        for (int i = tid; i < 2 * kTile * kAccDigits; i += blockDim.x) {
-            smem[i] = 0ull;
-        }
-        __syncthreads();
-
         if (tid == 0) {
             const long long now = clock64();
             atomicAdd(&cnts[kCyclesSssp], static_cast<unsigned long long>(now - t_phase));
@@ -933,8 +1027,10 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
             // ------------------------------------------------------------ shortest-path DAG: counts, sigma, delta
             // the level lists are built only after the successor lists: their storage holds pred[][] until then
             uint32_t* const pred = reinterpret_cast<uint32_t*>(list);
-            dag_count(g, rg, b.arc_src, b.m_total, n, nsrc, s_src, dist, tie, reinterpret_cast<unsigned long long*>(sigma), cnt, scnt, pred, lane,
-                      NGX_GW, NGX_GWARPS, &ctl()->active_pairs);
+            uint32_t* const low = stamp;  // its words held the distance phase's bounds until here
+            dag_low(dist, low, n, nsrc, lane, NGX_GW, NGX_GWARPS);
+            sync0();
+            dag_count(low, lane < nsrc ? s_src[lane] : -1, sigma, cnt, scnt, pred, &ctl()->active_pairs, NGX_GW);
             sync0();
             const unsigned long long dag_arcs = group_exclusive_scan(grp(), s, s_bar, scnt, soff, nt, s_part);
             const bool use_lists = dag_arcs <= static_cast<unsigned long long>(b.succ_capacity);
@@ -943,13 +1039,16 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
             }
             sync0();
             if (use_lists) {
-                dag_fill<kMode == kModeBrandes>(rg, b.arc_src, n, dist, cnt, pred, soff, scnt, succ, lane, NGX_GW, NGX_GWARPS);
+                dag_fill<kMode == kModeBrandes>(b.arc_src, low, cnt, pred, soff, scnt, succ, NGX_GW);
                 sync0();
                 dag_sort(soff, succ, nt, NGX_GT, NGX_GTHREADS);
             }
             if (!use_lists) {
                 for (int64_t i = NGX_GT; i < n; i += NGX_GTHREADS) {
-                    stamp[i] = 0u;  // its words held the distance phase's bounds until here
+                    stamp[i] = 0u;
+                }
+                for (int64_t i = NGX_GT; i < nt; i += NGX_GTHREADS) {
+                    lvl[i] = kNoLevel;
                 }
             }
             sync([&](volatile TileShared& c) {
@@ -975,8 +1074,10 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
                 const int v = s_src[lane];
                 if (v >= 0) {
                     const int64_t row = static_cast<int64_t>(v) * kTile + lane;
-                    lvl[row] = 0u;
                     sigma[row] = 1.0;
+                    if (!use_lists) {
+                        lvl[row] = 0u;
+                    }
                     if (use_lists) {
                         list[atomicAdd(&ctl()->lvl_len, 1)] = static_cast<int32_t>((static_cast<uint32_t>(v) << 5) | static_cast<uint32_t>(lane));
                     } else if (atomicExch(&stamp[v], s.stamp) != s.stamp) {
@@ -1001,8 +1102,8 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
                     dag_tree_level<kMode == kModeBrandes>(g, list + start, len, sigma, soff, succ, list + start + len, &ctl()->next_len, lane, NGX_GW,
                                                           NGX_GWARPS);
                 } else {
-                    dag_sigma_level<kMode == kModeBrandes>(g, list + start, len, level, sigma, cnt, lvl, soff, succ, list + start + len,
-                                                           &ctl()->next_len, b.sigma_inexact, lane, NGX_GW, NGX_GWARPS);
+                    dag_sigma_level<kMode == kModeBrandes>(g, list + start, len, sigma, cnt, soff, succ, list + start + len, &ctl()->next_len,
+                                                           b.sigma_inexact, lane, NGX_GW, NGX_GWARPS);
                 }
                 sync([&](volatile TileShared& c) {
                     c.lvl_start = start + len;
@@ -1031,11 +1132,6 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
                 }
                 sync0();
             }
-            // the pair buffers borrowed the epilogue's accumulators, which must start the epilogue at zero
-            for (int k = tid; k < (kBlock / 32) * 32 * delta_level_unroll(kMode) * (kMode == kModeGrad ? 2 : 1); k += blockDim.x) {
-                s_acc_sum[k] = 0ull;
-            }
-            __syncthreads();
             if (tid == 0) {
                 if ((!kMulti || grp().rank == 0)) {
                     atomicAdd(&cnts[kDagLevels], static_cast<unsigned long long>(levels));
@@ -1105,6 +1201,11 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
         }
 
         // ------------------------------------------------------------ epilogue: fused APSP summaries, reset
+        // the passes before borrowed the accumulators, which must start at zero (each ended with a barrier)
+        for (int i = tid; i < 2 * kTile * kAccDigits; i += blockDim.x) {
+            smem[i] = 0ull;
+        }
+        __syncthreads();
         const int my_src = s_src[lane];
         const bool valid = lane < nsrc;
         unsigned long long unreach = 0, arcs = 0, mx = 0, overflow = 0;
@@ -1145,17 +1246,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
                         fixed_add_parts(&bc_g[2 * v], lo, hi);
                     }
                 }
-                sigma[row] = __longlong_as_double(-1ll);
-                delta[row] = __longlong_as_double(-1ll);
-                if constexpr (kMode == kModeGrad) {
-                    delta_g[row] = 0.0;
-                }
-                cnt[row] = 0u;
-                lvl[row] = kNoLevel;
                 scnt[row] = 0u;
-                if (lane == 0) {
-                    tie[v] = 0u;
-                }
             }
             if (!valid) {
                 continue;
