@@ -115,6 +115,7 @@ struct TileShared {
     int lvl_len;
     int next_len;
     unsigned long long active_pairs;  // reached (vertex, source) pairs other than the sources, counted by the DAG pass
+    unsigned long long dag_arcs;      // DAG arcs of all the tile's sources, counted by the DAG pass
     int grab;                       // next queue entry handed to a warp in the current near iteration
     int touched_len;                // vertices the tile has reached so far (reach lists; see SsspParams::ws_touched)
     // the state of a CTA that left its group (ngx_group.cuh): no tile, nothing queued, pending or levelled
@@ -622,25 +623,28 @@ __device__ __forceinline__ void scan_in_arcs(const TileSmem& sh, WarpScratch& w,
 }
 
 // cnt[v][s] = DAG predecessors of (v, s), pred[v][s] = forward index of one of their arcs (the only one when cnt is 1),
-// scnt[u][s] += 1 for each DAG arc u -> v, sigma = 0; warp per vertex, lane per source. src_lane: this lane's source
-// vertex (-1 without one).
+// scnt[u][s] += 1 for each DAG arc u -> v, sigma = 0; warp per vertex, lane per source. parent[v][s] (unless nullptr) =
+// that arc's source. src_lane: this lane's source vertex (-1 without one).
 __device__ __noinline__ void dag_count(const uint32_t* low, int src_lane, double* sigma, uint32_t* cnt, uint32_t* scnt, uint32_t* pred,
-                                       unsigned long long* active_pairs, int gw) {
+                                       uint32_t* parent, TileShared* ctl, int gw) {
     extern __shared__ __align__(16) unsigned long long smem[];
     TileSmem& sh = *reinterpret_cast<TileSmem*>(smem);
     const int lane = threadIdx.x & 31;
     WarpScratch& w = sh.warp[threadIdx.x >> 5];
     unsigned active_count = 0;
+    unsigned arc_count = 0;
     for (int v = gw; v < sh.args.n; v += sh.args.group_warps) {
         const int64_t row = static_cast<int64_t>(v) * kTile + lane;
         const unsigned long long dv = __ldcg(&sh.args.dist[row]);
         const bool active = src_lane >= 0 && dv != kInfBits && v != src_lane;
         uint32_t c = 0;
         uint32_t first = 0;
+        int from = 0;
         if (__ballot_sync(kFullMask, active) != 0u) {
             active_count += active ? 1u : 0u;
             scan_in_arcs(sh, w, low, v, dv, active, lane, [&](int u, uint32_t e) {
                 first = c == 0 ? e : first;
+                from = u;
                 ++c;
                 atomicAdd(&scnt[static_cast<int64_t>(u) * kTile + lane], 1u);
             });
@@ -648,10 +652,81 @@ __device__ __noinline__ void dag_count(const uint32_t* low, int src_lane, double
         sigma[row] = 0.0;
         cnt[row] = c;
         pred[row] = first;
+        if (parent != nullptr) {
+            parent[row] = static_cast<uint32_t>(from);
+        }
+        arc_count += c;
     }
-    const unsigned total = __reduce_add_sync(kFullMask, active_count);
-    if (lane == 0 && total != 0u) {
-        atomicAdd(active_pairs, static_cast<unsigned long long>(total));
+    const unsigned pairs = __reduce_add_sync(kFullMask, active_count);
+    const unsigned long long arcs = __reduce_add_sync(kFullMask, arc_count & 0xFFFFu) +
+                                    (static_cast<unsigned long long>(__reduce_add_sync(kFullMask, arc_count >> 16)) << 16);
+    if (lane == 0 && arcs != 0ull) {
+        atomicAdd(&ctl->active_pairs, static_cast<unsigned long long>(pairs));
+        atomicAdd(&ctl->dag_arcs, arcs);
+    }
+}
+
+// Betweenness dependencies when every DAG of the tile is a tree (as many DAG arcs as reached non-source pairs, the rule
+// for tie-free weights). Every path count is 1, so delta[v][s] is the number of descendants of v: an integer, exact in
+// any order. acc[v][s] (zero before) gathers it from the leaves up in one atomic per pair: the low word sums
+// 1 + delta of the children, the high word counts the children done, and whoever adds the last child goes on with v. So
+// there are no lists, no levels and no barriers; the walks of a warp that go on wait in its scratch until 32 of them
+// make a full step. parent and scnt are those of dag_count, s_src the tile's sources.
+__device__ __noinline__ void dag_tree_walk(const uint32_t* cnt, const uint32_t* parent, const uint32_t* scnt, unsigned long long* acc,
+                                           const int* s_src, int gw) {
+    extern __shared__ __align__(16) unsigned long long smem[];
+    TileSmem& sh = *reinterpret_cast<TileSmem*>(smem);
+    const int lane = threadIdx.x & 31;
+    uint2* const stack = reinterpret_cast<uint2*>(sh.warp[threadIdx.x >> 5].kept);  // (v << 5 | s, delta), 256 entries
+    constexpr int kRows = 4;
+    static_assert(sizeof(Arc) * kArcBlock / sizeof(uint2) >= 32 * (kRows + 1), "a round's pushes fit on top of a partial step");
+    int waiting = 0;
+    // one child of (up, s) is done with `size` descendants and itself; pushes (up, s) when it was the last
+    const auto arrive = [&](bool on, uint32_t up, uint32_t s, uint32_t size) {
+        bool go_on = false;
+        uint32_t sum = 0;
+        if (on) {
+            const int64_t row = static_cast<int64_t>(up) * kTile + s;
+            const uint32_t children = __ldcg(&scnt[row]);
+            const unsigned long long old = atomicAdd(&acc[row], (1ull << 32) | (1ull + size));
+            sum = static_cast<uint32_t>(old) + 1u + size;
+            go_on = static_cast<uint32_t>(old >> 32) + 1u == children && static_cast<int>(up) != s_src[s];
+        }
+        const unsigned bal = __ballot_sync(kFullMask, go_on);
+        if (go_on) {
+            stack[waiting + __popc(bal & lanemask_lt())] = make_uint2(up << 5 | s, sum);
+        }
+        waiting += __popc(bal);
+        __syncwarp();
+    };
+    const auto step = [&](int take) {
+        waiting -= take;
+        const uint2 e = stack[waiting + (lane < take ? lane : 0)];
+        __syncwarp();
+        const uint32_t s = e.x & 31u;
+        const uint32_t up = lane < take ? __ldcg(&parent[static_cast<int64_t>(e.x >> 5) * kTile + s]) : 0u;
+        arrive(lane < take, up, s, e.y);
+    };
+    for (int v0 = gw; v0 < sh.args.n; v0 += kRows * sh.args.group_warps) {
+        bool leaf[kRows];
+        uint32_t up[kRows];
+#pragma unroll
+        for (int i = 0; i < kRows; ++i) {
+            const int64_t v = v0 + static_cast<int64_t>(i) * sh.args.group_warps;
+            const int64_t row = v * kTile + lane;
+            leaf[i] = v < sh.args.n && __ldcg(&cnt[row]) != 0u && __ldcg(&scnt[row]) == 0u;
+            up[i] = leaf[i] ? __ldcg(&parent[row]) : 0u;
+        }
+#pragma unroll
+        for (int i = 0; i < kRows; ++i) {
+            arrive(leaf[i], up[i], static_cast<uint32_t>(lane), 0u);
+        }
+        while (waiting >= 32) {
+            step(32);
+        }
+    }
+    while (waiting > 0) {
+        step(waiting < 32 ? waiting : 32);
     }
 }
 
@@ -856,6 +931,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
             c.iterations = 0;
             c.min_bits = kInfBits;
             c.active_pairs = 0;
+            c.dag_arcs = 0;
             c.grab = 0;
             c.touched_len = 0;
             if (c.tile < p.num_tiles) {
@@ -1023,6 +1099,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
             atomicAdd(&cnts[kCyclesSssp], static_cast<unsigned long long>(now - t_phase));
             t_phase = now;
         }
+        bool tree_walk = false;
         if constexpr (kMode != kModeApsp) {
             // ------------------------------------------------------------ shortest-path DAG: counts, sigma, delta
             // the level lists are built only after the successor lists: their storage holds pred[][] until then
@@ -1030,8 +1107,26 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
             uint32_t* const low = stamp;  // its words held the distance phase's bounds until here
             dag_low(dist, low, n, nsrc, lane, NGX_GW, NGX_GWARPS);
             sync0();
-            dag_count(low, lane < nsrc ? s_src[lane] : -1, sigma, cnt, scnt, pred, &ctl()->active_pairs, NGX_GW);
+            dag_count(low, lane < nsrc ? s_src[lane] : -1, sigma, cnt, scnt, pred, kMode == kModeBrandes ? lvl : nullptr, ctl(), NGX_GW);
             sync0();
+            tree_walk = kMode == kModeBrandes && s.dag_arcs == s.active_pairs && b.succ_capacity > 0;
+          if (tree_walk) {
+            if (tid == 0) {
+                const long long now = clock64();
+                atomicAdd(&cnts[kCyclesCount], static_cast<unsigned long long>(now - t_phase));
+                t_phase = now;
+            }
+            dag_tree_walk(cnt, lvl, scnt, reinterpret_cast<unsigned long long*>(sigma), s_src, NGX_GW);
+            sync0();
+            if (tid == 0) {
+                if (!kMulti || grp().rank == 0) {
+                    atomicAdd(&cnts[kDagEntries], s.active_pairs + static_cast<unsigned long long>(nsrc));
+                }
+                const long long now = clock64();
+                atomicAdd(&cnts[kCyclesDelta], static_cast<unsigned long long>(now - t_phase));
+                t_phase = now;
+            }
+          } else {
             const unsigned long long dag_arcs = group_exclusive_scan(grp(), s, s_bar, scnt, soff, nt, s_part);
             const bool use_lists = dag_arcs <= static_cast<unsigned long long>(b.succ_capacity);
             for (int64_t i = NGX_GT; i < nt; i += NGX_GTHREADS) {
@@ -1198,6 +1293,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
                 t_phase = now;
             }
           }
+          }
         }
 
         // ------------------------------------------------------------ epilogue: fused APSP summaries, reset
@@ -1236,14 +1332,25 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
                 const int64_t row = v * kTile + lane;
                 if constexpr (kMode == kModeBrandes) {
                     // BrandesVariant.h:156: every settled vertex but the source gains its dependency
-                    const double dep = (valid && v != my_src && bits != kInfBits) ? __ldcg(&delta[row]) : 0.0;
-                    // summed over the tile's sources in fixed point, exactly: betweenness does not depend on how
-                    // the sources are grouped into tiles
-                    unsigned long long lo, hi;
-                    fixed_parts(dep, lo, hi);
-                    fixed_warp_sum(lo, hi);
-                    if (lane == 0 && (lo | hi) != 0ull) {
-                        fixed_add_parts(&bc_g[2 * v], lo, hi);
+                    const bool gains = valid && v != my_src && bits != kInfBits;
+                    if (tree_walk) {
+                        // integers (descendant counts): exact in double and in fixed point alike
+                        const unsigned long long dep = gains ? __ldcg(reinterpret_cast<unsigned long long*>(&sigma[row])) & 0xFFFFFFFFull : 0ull;
+                        const unsigned long long sum = __reduce_add_sync(kFullMask, static_cast<unsigned>(dep & 0xFFFFull)) +
+                                                       (static_cast<unsigned long long>(__reduce_add_sync(kFullMask, static_cast<unsigned>(dep >> 16))) << 16);
+                        if (lane == 0 && sum != 0ull) {
+                            atomicAdd(&bc_g[2 * v + 1], sum);
+                        }
+                    } else {
+                        const double dep = gains ? __ldcg(&delta[row]) : 0.0;
+                        // summed over the tile's sources in fixed point, exactly: betweenness does not depend on how
+                        // the sources are grouped into tiles
+                        unsigned long long lo, hi;
+                        fixed_parts(dep, lo, hi);
+                        fixed_warp_sum(lo, hi);
+                        if (lane == 0 && (lo | hi) != 0ull) {
+                            fixed_add_parts(&bc_g[2 * v], lo, hi);
+                        }
                     }
                 }
                 scnt[row] = 0u;
