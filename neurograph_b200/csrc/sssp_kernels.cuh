@@ -101,12 +101,12 @@ struct TileShared {
     long long tile;
     int qlen[2];
     int cur;
+    int bucket_len;                 // bucket step: entries pushed so far (qlen[cur] is still being read as 0 by late warps)
     int stop;
     unsigned stamp;                 // id of the DAG pass about to run (dedup of its level lists)
-    int done;                       // bucket step: no pending far pair is left
     double theta;
-    double theta_next;              // bucket step: the bound below which pass 2 moves pairs to the near queue
-    unsigned long long min_bits;
+    unsigned long long min_bits;    // a lower bound of the smallest pending far distance (+inf: none is pending)
+    unsigned long long min_left;    // bucket step: smallest far distance that stays far
     unsigned long long iterations;
     unsigned long long overflow;    // histogram overflow of the tile (plain form)
     // Brandes / adjoint levels
@@ -124,7 +124,7 @@ struct TileShared {
         tile = 0x7FFFFFFFFFFFFFFFll;
         qlen[0] = 0;
         qlen[1] = 0;
-        done = 1;
+        min_bits = kInfBits;
         level = 0u;
         lvl_start = 0;
         lvl_len = 0;
@@ -151,12 +151,27 @@ __device__ __forceinline__ Group<TileShared> tile_group(const Params& p, TileSha
                               static_cast<int>(blockIdx.x % p.group_size), p.error };
 }
 
+// Smallest of the lanes' values, in every lane.
+__device__ __forceinline__ unsigned long long warp_min(unsigned long long x) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        const unsigned long long o = __shfl_xor_sync(kFullMask, x, off);
+        x = o < x ? o : x;
+    }
+    return x;
+}
+
 // Queue entries a warp takes at a time (guided self-scheduling): the entries not yet handed out over twice the group's
-// warps, clamped to 1..32, so a near iteration starts with large chunks (one round of loads serves many entries) and
-// ends with single entries (a vertex expansion takes tens of microseconds: a coarse last chunk would leave the other
-// warps of the group waiting at the barrier that closes the iteration).
-__device__ __forceinline__ int expand_chunk(int remaining, int group_warps) {
-    const int c = remaining / (2 * group_warps);
+// warps, clamped to 1..32, so a near iteration starts with large chunks (one round of loads serves many entries) and ends
+// with single entries (an expansion can be work for a whole warp: a coarse last chunk would leave the other warps of
+// the group waiting at the barrier that closes the iteration). Where entries are small (mean out-degree below
+// kFilterDegree) packed_expand works several in the time of one, and a warp takes its whole share, up to 8, at once.
+__device__ __forceinline__ int expand_chunk(int remaining, int group_warps, bool small_entries) {
+    int c = remaining / (2 * group_warps);
+    if (small_entries && c < 8) {
+        const int share = remaining / group_warps;
+        c = share < 8 ? share : 8;
+    }
     return c < 1 ? 1 : (c > 32 ? 32 : c);
 }
 
@@ -200,6 +215,10 @@ struct WarpWork {
     unsigned long long lane_expansions;
 };
 
+// Near iterations between two looks at the abort flag: it lies in host memory, and the read (about a microsecond over
+// PCIe) would be on the path of every iteration's barrier. A power of two.
+constexpr unsigned long long kAbortPoll = 8;
+
 constexpr int kMaxWarps = 16;
 constexpr int kAccBytes = 2 * kTile * kAccDigits * 8;
 
@@ -220,12 +239,13 @@ struct ExpandArgs {
     int bound_base;
     int group_warps;
     int n;
+    int small_entries;
 };
 
 // Dynamic shared memory of the tile kernel, before the histogram. The distance phase's warp scratch overlays the
 // epilogue's accumulators (2 x kTile x kAccDigits words, zero outside the distance phase) and, after them, the scan
 // partials of the DAG phase.
-struct TileSmem {
+struct __align__(16) TileSmem {
     WarpScratch warp[kMaxWarps];
     WarpWork work[kMaxWarps];
     ExpandArgs args;
@@ -240,7 +260,7 @@ static_assert(sizeof(TileSmem) % 16 == 0, "the histogram follows");
 // finite distance of (x, s) appends x to the tile's reached vertices.
 template <int kUnroll, bool kReach>
 __device__ __forceinline__ void relax_lane(const int (&x)[kUnroll], int src, const double (&nd)[kUnroll], const unsigned long long (&cur)[kUnroll],
-                                           unsigned long long* dist_s, const TileSmem& sh) {
+                                           unsigned long long* dist_s, const TileSmem& sh, unsigned long long& far_min) {
 #pragma unroll
     for (int u = 0; u < kUnroll; ++u) {
         const unsigned long long nb = static_cast<unsigned long long>(__double_as_longlong(nd[u]));
@@ -255,7 +275,12 @@ __device__ __forceinline__ void relax_lane(const int (&x)[kUnroll], int src, con
             if (kReach && cur[u] == kInfBits) {
                 sh.args.reach.add(x[u], bit);
             }
-            const uint32_t which = nd[u] < sh.ctl.theta ? static_cast<uint32_t>(sh.ctl.cur ^ 1) : 2u;
+            uint32_t which = static_cast<uint32_t>(sh.ctl.cur ^ 1);
+            if (!(nd[u] < sh.ctl.theta)) {
+                which = 2u;
+                const unsigned long long nb = static_cast<unsigned long long>(__double_as_longlong(nd[u]));
+                far_min = nb < far_min ? nb : far_min;
+            }
             atomicOr(&sh.args.marks[static_cast<size_t>(which) * sh.args.n_slot + static_cast<uint32_t>(x[u])], bit);
         }
     }
@@ -307,7 +332,7 @@ constexpr int kFilterDegree = 16;
 // The caller has taken v's pending mask (entry.mask, non-zero) and cleared it and v's superseded far marks: see
 // expand_queue. Lanes >= nsrc hold no source.
 template <int kUnroll, bool kReach>
-__device__ __forceinline__ void batched_expand(TileSmem& sh, WarpScratch& w, WarpWork& work, int j, int lane) {
+__device__ __forceinline__ void batched_expand(TileSmem& sh, WarpScratch& w, WarpWork& work, int j, int lane, unsigned long long& far_min) {
     const QueueEntry entry = w.entry[j];
     const uint32_t amask = entry.mask;
     unsigned long long* const dist = sh.args.dist;
@@ -385,7 +410,7 @@ __device__ __forceinline__ void batched_expand(TileSmem& sh, WarpScratch& w, War
                 cur[u] = __ldcg(&dist_s[static_cast<int64_t>(x[u]) * kTile]);
                 a += step_a;
             }
-            relax_lane<kUnroll, kReach>(x, src, nd, cur, dist_s, sh);
+            relax_lane<kUnroll, kReach>(x, src, nd, cur, dist_s, sh, far_min);
         }
         __syncwarp();  // the next block of arcs (the next vertex) overwrites kept (and rank)
     }
@@ -393,10 +418,7 @@ __device__ __forceinline__ void batched_expand(TileSmem& sh, WarpScratch& w, War
 
 // Queue entries with fewer (arc, pending source) pairs than this leave most of a warp idle in batched_expand (32 lanes,
 // several arcs per lane in flight); consecutive ones are expanded together by packed_expand.
-#ifndef NGX_PACK_PAIRS
-#define NGX_PACK_PAIRS 64
-#endif
-constexpr int kPackPairs = NGX_PACK_PAIRS;
+constexpr int kPackPairs = 64;
 
 // Expands a group of m small queue entries together: w.rank[t], t < ktot <= 32, names the t-th (entry, pending source) of
 // the group. Lane t takes it and walks its entry's arcs, kUnroll at a time: the lanes of an entry read the same arc
@@ -404,7 +426,8 @@ constexpr int kPackPairs = NGX_PACK_PAIRS;
 // its entry with the most arcs. The relaxations and the counters are batched_expand's; the arcs are not filtered (a bound read per arc would cost as much as the few distance reads it
 // saves).
 template <int kUnroll, bool kReach>
-__device__ __forceinline__ void packed_expand(TileSmem& sh, WarpScratch& w, WarpWork& work, int m, int ktot, int lane) {
+__device__ __forceinline__ void packed_expand(TileSmem& sh, WarpScratch& w, WarpWork& work, int m, int ktot, int lane,
+                                              unsigned long long& far_min) {
     const int code = w.rank[lane < ktot ? lane : 0];
     const int src = code & 31;
     const QueueEntry entry = w.entry[code >> 5];
@@ -433,7 +456,7 @@ __device__ __forceinline__ void packed_expand(TileSmem& sh, WarpScratch& w, Warp
             nd[u] = a < deg ? __dadd_rn(dvs, arc.len) : INFINITY;
             cur[u] = __ldcg(&dist_s[static_cast<int64_t>(x[u]) * kTile]);
         }
-        relax_lane<kUnroll, kReach>(x, src, nd, cur, dist_s, sh);
+        relax_lane<kUnroll, kReach>(x, src, nd, cur, dist_s, sh, far_min);
     }
 }
 
@@ -443,12 +466,13 @@ __device__ __forceinline__ void packed_expand(TileSmem& sh, WarpScratch& w, Warp
 // vertex has a loop iteration's worth of (arc, source) pairs or more, else with its small neighbours in the chunk.
 // Not inlined: the registers of the other phases are saved around the call instead of being spilled inside its loops.
 template <int kUnroll, bool kReach>
-__device__ __noinline__ void expand_queue() {
+__device__ __noinline__ void expand_queue(unsigned long long* min_bits) {
     extern __shared__ __align__(16) unsigned long long smem[];
     TileSmem& sh = *reinterpret_cast<TileSmem*>(smem);
     const int lane = threadIdx.x & 31;
     WarpScratch& w = sh.warp[threadIdx.x >> 5];
     WarpWork& work = sh.work[threadIdx.x >> 5];
+    unsigned long long far_min = kInfBits;
     for (;;) {
         int base = 0;
         int chunk = 0;
@@ -457,7 +481,7 @@ __device__ __noinline__ void expand_queue() {
             // the grab counter is in shared memory for single-CTA tiles and in global memory for groups: a volatile
             // generic load reads either (for global memory, from L2)
             int* const grab = sh.args.grab;
-            chunk = expand_chunk(qlen - *reinterpret_cast<volatile int*>(grab), sh.args.group_warps);
+            chunk = expand_chunk(qlen - *reinterpret_cast<volatile int*>(grab), sh.args.group_warps, sh.args.small_entries != 0);
             base = atomicAdd(grab, chunk);
         }
         base = __shfl_sync(kFullMask, base, 0);
@@ -529,16 +553,20 @@ __device__ __noinline__ void expand_queue() {
                     const int last_lane = 31 - __clz(fit);
                     const int ktot = __shfl_sync(kFullMask, kin, last_lane);
                     __syncwarp();
-                    packed_expand<kUnroll, kReach>(sh, w, work, m, ktot, lane);
+                    packed_expand<kUnroll, kReach>(sh, w, work, m, ktot, lane, far_min);
                     __syncwarp();  // the next group overwrites rank
                     j = last_lane + 1;
                     continue;
                 }
             }
-            batched_expand<kUnroll, kReach>(sh, w, work, j, lane);
+            batched_expand<kUnroll, kReach>(sh, w, work, j, lane, far_min);
             ++j;
         }
         __syncwarp();  // the next chunk overwrites the entries
+    }
+    far_min = warp_min(far_min);
+    if (lane == 0 && far_min != kInfBits) {
+        atomicMin(min_bits, far_min);
     }
 }
 
@@ -924,12 +952,17 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
             }
             c.tile = static_cast<long long>(atomicAdd(p.tile_counter, 1ull));
             c.stop = *reinterpret_cast<volatile int*>(p.error) != 0 ? 1 : 0;
+            if (*p.abort_flag != 0) {
+                atomicCAS(p.error, kDevOk, kDevAborted);
+                c.stop = 1;
+            }
             c.qlen[0] = 0;
             c.qlen[1] = 0;
             c.cur = 0;
-            c.done = 0;
+            c.bucket_len = 0;
             c.iterations = 0;
             c.min_bits = kInfBits;
+            c.min_left = kInfBits;
             c.active_pairs = 0;
             c.dag_arcs = 0;
             c.grab = 0;
@@ -967,7 +1000,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
         if (tid == 0) {
             sh.args = ExpandArgs{ g.arcs, g.row_ptr, rg.arcs, rg.row_ptr, dist, pend0, q0, bound, &ctl()->grab, reach,
                                   static_cast<uint32_t>(n_slot), nsrc, static_cast<int>(static_cast<uint32_t>(__double2hiint(0.25 * gd.delta)) >> 15),
-                                  NGX_GWARPS, static_cast<int>(n) };
+                                  NGX_GWARPS, static_cast<int>(n), gd.m < kFilterDegree * gd.n ? 1 : 0 };
         }
         __syncthreads();
         if ((!kMulti || grp().rank == 0) && warp == 0) {
@@ -996,7 +1029,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
                 }
                 uint32_t* pend_nxt = cur ? pend0 : pend1;
                 int32_t* q_nxt = cur ? q0 : q1;
-                expand_queue<kUnroll, kReach>();
+                expand_queue<kUnroll, kReach>(&ctl()->min_bits);
                 sync([&](volatile TileShared& c) {
                     c.qlen[cur] = 0;
                     c.grab = 0;
@@ -1004,7 +1037,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
                     if (c.iterations > p.max_iterations) {
                         atomicCAS(p.error, kDevOk, kDevTimeout);
                         c.stop = 1;
-                    } else if (*p.abort_flag != 0) {
+                    } else if ((c.iterations & (kAbortPoll - 1)) == 0 && *p.abort_flag != 0) {
                         atomicCAS(p.error, kDevOk, kDevAborted);
                         c.stop = 1;
                     }
@@ -1020,75 +1053,70 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
             if (s.stop != 0) {
                 break;
             }
-            // bucket step, pass 1: smallest pending far distance (min_bits is +inf here: reset at the tile's start and
-            // after every bucket step)
-            // (over the tile's reached vertices when it keeps a reach list: no other vertex has far marks)
+            // bucket step: no near work is left. Every far mark set since the last step offered its distance to min_bits, and
+            // that step left the smallest distance it kept far there, so the next bound needs no pass of its own. (A mark
+            // that has been superseded may make it too low: the step then moves nothing and leaves the true minimum.)
+            if (s.min_bits == kInfBits) {
+                break;  // nothing pending: the tile's distances are final
+            }
+            const double theta = next_theta(__longlong_as_double(static_cast<long long>(s.min_bits)), gd.delta);
+            // one pass over the far marks (of the tile's reached vertices when it keeps a reach list: no other vertex has
+            // any) moves the pairs below the new bound into the near queue of the next iteration
             const int64_t span = kReach ? static_cast<int64_t>(s.touched_len) : n;
-            unsigned long long local_min = kInfBits;
-            for (int64_t vb = static_cast<int64_t>(NGX_GW) * 32; vb < span; vb += static_cast<int64_t>(NGX_GWARPS) * 32) {
-                const int64_t i = vb + lane;
-                const int64_t v = i < span ? (kReach ? static_cast<int64_t>(__ldcg(&reach.list[i])) : i) : 0;
-                const uint32_t fm = i < span ? __ldcg(&far[v]) : 0u;
-                unsigned any = __ballot_sync(kFullMask, fm != 0u);
-                while (any != 0u) {
-                    const int l = __ffs(any) - 1;
-                    any &= any - 1u;
-                    const uint32_t f = __shfl_sync(kFullMask, fm, l);
-                    const int64_t vl = __shfl_sync(kFullMask, v, l);
-                    if ((f >> lane) & 1u) {
-                        const unsigned long long d = __ldcg(&dist[vl * kTile + lane]);
-                        local_min = d < local_min ? d : local_min;
-                    }
-                }
-            }
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) {
-                const unsigned long long o = __shfl_xor_sync(kFullMask, local_min, off);
-                local_min = o < local_min ? o : local_min;
-            }
-            if (lane == 0 && local_min != kInfBits) {
-                atomicMin(&ctl()->min_bits, local_min);
-            }
-            sync([&](volatile TileShared& c) {
-                if (c.min_bits == kInfBits) {
-                    c.done = 1;  // nothing pending: the tile's distances are final
-                } else {
-                    c.theta_next = next_theta(__longlong_as_double(static_cast<long long>(c.min_bits)), gd.delta);
-                }
-            });
-            if (s.done != 0) {
-                break;
-            }
-            const double theta = s.theta_next;
-            // pass 2: move the pairs below the new bound into the near queue of the next iteration
             const int cur = s.cur;
             uint32_t* pend_cur = cur ? pend1 : pend0;
             int32_t* q_cur = cur ? q1 : q0;
+            unsigned long long left = kInfBits;
             for (int64_t vb = static_cast<int64_t>(NGX_GW) * 32; vb < span; vb += static_cast<int64_t>(NGX_GWARPS) * 32) {
                 const int64_t i = vb + lane;
                 const int64_t v = i < span ? (kReach ? static_cast<int64_t>(__ldcg(&reach.list[i])) : i) : 0;
                 const uint32_t fm = i < span ? __ldcg(&far[v]) : 0u;
                 unsigned any = __ballot_sync(kFullMask, fm != 0u);
+                uint32_t moved = 0u;  // this lane's vertex: sources that move
                 while (any != 0u) {
-                    const int l = __ffs(any) - 1;
+                    // two marked vertices at a time, their rows read side by side
+                    const int l0 = __ffs(any) - 1;
                     any &= any - 1u;
-                    const uint32_t f = __shfl_sync(kFullMask, fm, l);
-                    const int64_t vv = __shfl_sync(kFullMask, v, l);
-                    bool near = false;
-                    if ((f >> lane) & 1u) {
-                        near = __longlong_as_double(static_cast<long long>(__ldcg(&dist[vv * kTile + lane]))) < theta;
+                    const int l1 = any != 0u ? __ffs(any) - 1 : l0;
+                    any &= any - 1u;
+                    const uint32_t f0 = __shfl_sync(kFullMask, fm, l0);
+                    const uint32_t f1 = __shfl_sync(kFullMask, fm, l1);
+                    const int64_t v0 = __shfl_sync(kFullMask, v, l0);
+                    const int64_t v1 = __shfl_sync(kFullMask, v, l1);
+                    const unsigned long long d0 = (f0 >> lane) & 1u ? __ldcg(&dist[v0 * kTile + lane]) : kInfBits;
+                    const unsigned long long d1 = (f1 >> lane) & 1u ? __ldcg(&dist[v1 * kTile + lane]) : kInfBits;
+                    const bool near0 = __longlong_as_double(static_cast<long long>(d0)) < theta;
+                    const bool near1 = __longlong_as_double(static_cast<long long>(d1)) < theta;
+                    left = !near0 && d0 < left ? d0 : left;
+                    left = !near1 && d1 < left ? d1 : left;
+                    const unsigned n0 = __ballot_sync(kFullMask, near0);
+                    const unsigned n1 = __ballot_sync(kFullMask, near1);
+                    moved = lane == l0 ? n0 : (lane == l1 ? n1 : moved);
+                }
+                const unsigned bal = __ballot_sync(kFullMask, moved != 0u);
+                if (bal != 0u) {
+                    int qb = 0;
+                    if (lane == 0) {
+                        qb = atomicAdd(&ctl()->bucket_len, __popc(bal));
                     }
-                    const unsigned nmask = __ballot_sync(kFullMask, near);
-                    if (nmask != 0u && lane == 0) {
-                        far[vv] = f & ~nmask;
-                        pend_cur[vv] = nmask;
-                        q_cur[atomicAdd(&ctl()->qlen[cur], 1)] = static_cast<int32_t>(vv);
+                    qb = __shfl_sync(kFullMask, qb, 0);
+                    if (moved != 0u) {
+                        far[v] = fm & ~moved;
+                        pend_cur[v] = moved;
+                        q_cur[qb + __popc(bal & lanemask_lt())] = static_cast<int32_t>(v);
                     }
                 }
             }
+            left = warp_min(left);
+            if (lane == 0 && left != kInfBits) {
+                atomicMin(&ctl()->min_left, left);
+            }
             sync([&](volatile TileShared& c) {
-                c.theta = c.theta_next;
-                c.min_bits = kInfBits;
+                c.qlen[cur] = c.bucket_len;
+                c.bucket_len = 0;
+                c.theta = theta;
+                c.min_bits = c.min_left;
+                c.min_left = kInfBits;
             });
         }
         if (s.stop != 0) {
