@@ -153,6 +153,7 @@ int time_wave(ngx_graph* g, int mode, int32_t gi, double scale, const ngx_apsp_o
         job.d_items = d_items;
         job.num_sources = part.n;
         job.n_max = g->n;
+        job.num_arcs = part.m_stored;
         float ms = 0.0f;
         rc = launch_tiles(g, &aopts, mode, job, 0, 0.0, o, mode != kModeApsp ? &extra : nullptr, &ms, true);
         if (rc == NGX_OK) {
@@ -294,6 +295,7 @@ int ngx_batch_run(ngx_graph* g, const ngx_batch_opts* opts, ngx_apsp_result* res
         job.d_items = static_cast<const WorkItem*>(g->d_items);
         job.num_sources = g->n_total;
         job.n_max = g->n;
+        job.num_arcs = g->m_stored;
         job.plain_delta = 1.0;
 
         const uint64_t key = options_key(opts, g);

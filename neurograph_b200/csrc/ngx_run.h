@@ -40,6 +40,7 @@ struct TileJob {
     const WorkItem* d_items = nullptr; // nullptr: tile t of graph 0
     int64_t num_sources = 0;
     int64_t n_max = 0;                 // largest graph (workspace slot size)
+    int64_t num_arcs = 0;              // stored arcs of the job's graphs
     double plain_delta = 1.0;          // bucket width of the plain form (single graph)
     bool track_reach = false;          // keep per-tile reach lists (a graph of several strongly connected components)
 };

@@ -184,25 +184,35 @@ const void* tile_kernel_for_block(int block, int ctas_per_sm, bool reach, bool m
     }
 }
 
-// CTAs per tile group: the caller's choice, else the largest of three needs.
-//  * L2 residency: the distance phase of a tile touches about 280 bytes per vertex (its 256-byte distance rows, pending
-//    marks, queues); when a tile fits in L2, as many tiles are kept in flight as fit in 90 % of it, each worked by
-//    resident / that many CTAs (measured: 4 tiles of 74 CTAs on the 100,000-vertex connectome, +20 % for APSP and
-//    +18 % for Brandes over one CTA per tile).
-//  * Few tiles: a run with fewer tiles than resident CTAs gives each tile the CTAs the others would leave idle.
+// CTAs per tile group: the caller's choice, else by the sizes of the job's graphs and its number of tiles.
+//  * Work per phase. A tile's phases (near iterations, bucket steps, DAG passes) end with a barrier of its group, and the
+//    entries of a phase grow with n while their number grows slowly, so larger graphs feed more CTAs: about
+//    0.12 sqrt(n), as many tiles in flight as then fit in the resident CTAs, at least four. Measured kernel times
+//    (Brandes unless noted, CTAs per tile: ms): n = 1e4, degree 40: 3: 79, 7: 62, 10-14: 58, 24: 66; n = 2e4, degree 6:
+//    1: 267, 4: 217, 14: 197; n = 3e4, degree 40: 7: 183, 21: 152, 42: 156; n = 5e4 (gradient): 9: 73, 18-37: 67, 49: 69;
+//    n = 1e5, degree 100 (APSP): 37-49: 176, 74: 179, 148: 234; n = 3e5, degree 40: 4: 337, 37-74: 264, 100: 325;
+//    n = 1e6: 18: 309, 74: 279; batches of mixed graphs, mean n 800: 1: 19.3, 2: 16.4, 8: 29; 3200: 1: 138, 6: 127, 11: 156;
+//    13,400: 1: 637, 11: 522, 24: 581. Keeping the tiles in flight within L2 matters less: the rate of random sector
+//    reads halves between 65 and 100 MB (microbenchmark), but the barriers of larger groups cost more than that.
+//  * Few tiles: a run with fewer tiles than resident CTAs gives each tile the CTAs the others would leave idle, up to five
+//    times the above (n = 2e4, 2 tiles: 37: 1.22, 74: 0.94, 148: 1.05 ms; n = 300, 10 tiles: 4: 0.49, 8-16: 0.45).
+//  * Sparse graphs (mean out-degree below 4) have long shortest paths, so many phases with few entries each: one CTA per
+//    tile while there are two tiles for every resident CTA (n = 2e4, degree 2, 626 tiles: 1: 70, 3: 75, 7: 92, 14: 118 ms),
+//    more in proportion when there are fewer.
 //  * Memory: when the device affords fewer workspace slots than that, each slot gets enough CTAs to use every SM.
-int choose_group_size(int requested, int64_t resident, int64_t num_tiles, int64_t affordable_slots, int64_t n, size_t l2_bytes) {
+int choose_group_size(int requested, int64_t resident, int64_t num_tiles, int64_t affordable_slots, double typical_n, double mean_degree) {
     if (requested > 0) {
         return static_cast<int>(std::min<int64_t>({ static_cast<int64_t>(requested), resident, static_cast<int64_t>(kMaxGroupSize) }));
     }
-    int64_t group = 1;
-    const double tile_bytes = 280.0 * static_cast<double>(std::max<int64_t>(n, 1));
-    const double room = 0.9 * static_cast<double>(l2_bytes);
-    if (tile_bytes <= 0.5 * room) {
-        const int64_t in_flight = std::max<int64_t>(1, static_cast<int64_t>(room / tile_bytes));
-        group = std::max<int64_t>(group, resident / in_flight);
+    const double wanted = 0.12 * std::sqrt(std::max(typical_n, 1.0));
+    int64_t in_flight = static_cast<int64_t>(static_cast<double>(resident) / std::max(wanted, 1.0) + 0.5);
+    in_flight = std::max<int64_t>(in_flight, 4);
+    int64_t group = std::max<int64_t>(1, resident / in_flight);
+    if (mean_degree < 4.0) {
+        group = std::min(group, std::max<int64_t>(1, 2 * resident / std::max<int64_t>(1, num_tiles)));
     }
-    group = std::max<int64_t>(group, resident / std::max<int64_t>(1, num_tiles));
+    const int64_t idle_share = resident / std::max<int64_t>(1, num_tiles);
+    group = std::max(group, std::min(idle_share, static_cast<int64_t>(5.0 * wanted)));
     if (affordable_slots < std::min(resident, num_tiles)) {
         // enough CTAs per slot that the affordable slots hold every resident CTA (rounded up: the slot count then
         // follows from the group size, and no CTA is left without a slot)
@@ -278,9 +288,12 @@ int launch_tiles(ngx_graph* g, const ngx_apsp_opts* opts, int tile_mode, const T
     const size_t dag_bytes = tile_mode == kModeApsp ? 0 : batched ? brandes_slot_bytes(n, tile_mode == kModeGrad) : plain_brandes_slot_bytes(n);
     const size_t data_bytes = sssp_slot_bytes(n, width) + dag_bytes + reach_bytes;
     const size_t budget = workspace_budget(g);
+    // the sizes the group rule goes by: the graph's, or the mean over a batch's graphs
+    const double typical_n = job.num_graphs > 1 ? static_cast<double>(g->n_total) / static_cast<double>(job.num_graphs) : static_cast<double>(n);
+    const double mean_degree = static_cast<double>(job.num_arcs) / std::max(1.0, typical_n * static_cast<double>(job.num_graphs));
     // the group size decides the group storage per slot, which the slot count must leave room for
     const int64_t affordable = static_cast<int64_t>(budget / (data_bytes + static_cast<size_t>(group_stride_words(kMaxGroupSize)) * 8));
-    const int group = batched && default_shape ? choose_group_size(opts->tile_ctas, resident, num_tiles, affordable, n, g->l2_bytes) : 1;
+    const int group = batched && default_shape ? choose_group_size(opts->tile_ctas, resident, num_tiles, affordable, typical_n, mean_degree) : 1;
     if (group > 1) {
         kernel = pick(track, true);  // the same shape and occupancy, built for groups
         NGX_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
@@ -637,6 +650,7 @@ int run_sources(ngx_graph* g, const ngx_apsp_opts* opts, int tile_mode, const st
     job.d_items = nullptr;
     job.num_sources = num_sources;
     job.n_max = part.n;
+    job.num_arcs = part.m_stored;
     job.plain_delta = delta;
     job.track_reach = g->scc_components > 1;
     return launch_tiles(g, opts, tile_mode, job, hist_bins, hist_max, o, extra, ms, true);
