@@ -549,60 +549,7 @@ int ngx_graph_update_weights(ngx_graph* g, const double* w) {
             return fail(NGX_INVALID_ARGUMENT, "ngx_graph_update_weights: graph or w is NULL");
         }
         NGX_CUDA_TRY(cudaSetDevice(g->device));
-        if (const int rc = ensure_stored_of_user(g); rc != NGX_OK) {
-            return rc;
-        }
-        const size_t m = static_cast<size_t>(g->m_stored);
-        std::vector<Arc> regular(m), inverse(m), rarcs(m);
-        NGX_CUDA_TRY(cudaStreamSynchronize(g->stream));
-        NGX_CUDA_TRY(cudaMemcpy(regular.data(), g->d_arcs_regular, m * sizeof(Arc), cudaMemcpyDeviceToHost));
-        NGX_CUDA_TRY(cudaMemcpy(rarcs.data(), g->d_rarcs, m * sizeof(Arc), cudaMemcpyDeviceToHost));
-        for (int64_t e = 0; e < g->m_user; ++e) {
-            const int32_t stored = g->stored_of_user[static_cast<size_t>(e)];
-            const double a = std::fabs(w[e]);
-            if (!std::isfinite(w[e]) || (stored < 0) != (a == 0.0)) {
-                return fail(NGX_INVALID_ARGUMENT, "ngx_graph_update_weights: arc " + std::to_string(e) + " is non-finite or changes between zero and non-zero");
-            }
-            if (stored >= 0) {
-                regular[static_cast<size_t>(stored)].len = a;
-            }
-        }
-        double sum_regular = 0.0, sum_inverse = 0.0, min_regular = INFINITY, max_regular = 0.0;
-        for (size_t e = 0; e < m; ++e) {
-            inverse[e] = regular[e];
-            inverse[e].len = 1.0 / regular[e].len;
-            sum_regular += regular[e].len;
-            sum_inverse += inverse[e].len;
-            min_regular = std::min(min_regular, regular[e].len);
-            max_regular = std::max(max_regular, regular[e].len);
-        }
-        for (size_t r = 0; r < m; ++r) {
-            rarcs[r].len = regular[static_cast<size_t>(rarcs[r].id)].len;
-        }
-        for (GraphPart& part : g->parts) {
-            double sr = 0.0, si = 0.0;
-            for (int64_t e = 0; e < part.m_user; ++e) {
-                const int32_t stored = g->stored_of_user[static_cast<size_t>(part.user_arc_off + e)];
-                if (stored >= 0) {
-                    sr += regular[static_cast<size_t>(stored)].len;
-                    si += inverse[static_cast<size_t>(stored)].len;
-                }
-            }
-            if (part.m_stored > 0) {
-                part.mean_len_regular = sr / static_cast<double>(part.m_stored);
-                part.mean_len_inverse = si / static_cast<double>(part.m_stored);
-            }
-        }
-        if (m > 0) {
-            g->mean_len_regular = sum_regular / static_cast<double>(m);
-            g->mean_len_inverse = sum_inverse / static_cast<double>(m);
-            g->min_len_regular = min_regular;
-            g->max_len_regular = max_regular;
-            NGX_CUDA_TRY(cudaMemcpy(g->d_arcs_regular, regular.data(), m * sizeof(Arc), cudaMemcpyHostToDevice));
-            NGX_CUDA_TRY(cudaMemcpy(g->d_arcs_inverse, inverse.data(), m * sizeof(Arc), cudaMemcpyHostToDevice));
-            NGX_CUDA_TRY(cudaMemcpy(g->d_rarcs, rarcs.data(), m * sizeof(Arc), cudaMemcpyHostToDevice));
-        }
-        return NGX_OK;
+        return update_weights_on_device(g, w);
     });
 }
 

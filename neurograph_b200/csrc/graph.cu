@@ -712,20 +712,6 @@ int ensure_source_order(ngx_graph* g) {
     return ensure_source_order(g);  // then grouped by component
 }
 
-int ensure_stored_of_user(ngx_graph* g) {
-    if (static_cast<int64_t>(g->stored_of_user.size()) == g->m_user || g->d_stored_of_user == nullptr) {
-        return NGX_OK;
-    }
-    HostVector<int32_t> map(static_cast<size_t>(g->m_user));
-    NGX_CUDA_TRY(cudaSetDevice(g->device));
-    if (!map.empty()) {
-        NGX_CUDA_TRY(cudaMemcpyAsync(map.data(), g->d_stored_of_user, map.size() * 4, cudaMemcpyDeviceToHost, g->stream));
-        NGX_CUDA_TRY(cudaStreamSynchronize(g->stream));
-    }
-    g->stored_of_user = std::move(map);
-    return NGX_OK;
-}
-
 }  // namespace ngx
 
 using namespace ngx;

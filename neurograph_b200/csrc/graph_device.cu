@@ -126,6 +126,52 @@ __global__ void reverse_records_kernel(const int32_t* __restrict__ sorted_index,
     }
 }
 
+// Checks new weights against the stored arcs: the smallest caller arc that is not finite or changes between zero and
+// non-zero, and the range of the new lengths.
+__global__ void check_weights_kernel(const double* __restrict__ w, const int32_t* __restrict__ stored_of_user, int64_t m_user,
+                                     unsigned long long* bad_arc, unsigned long long* min_len_bits, unsigned long long* max_len_bits) {
+    unsigned long long lo = ~0ull, hi = 0ull, bad = ~0ull;
+    for (int64_t e = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; e < m_user; e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+        const double a = fabs(w[e]);
+        if (!isfinite(a) || (stored_of_user[e] < 0) != (a == 0.0)) {
+            bad = static_cast<unsigned long long>(e) < bad ? static_cast<unsigned long long>(e) : bad;
+        } else if (a != 0.0) {
+            const unsigned long long bits = static_cast<unsigned long long>(__double_as_longlong(a));
+            lo = bits < lo ? bits : lo;
+            hi = bits > hi ? bits : hi;
+        }
+    }
+    if (bad != ~0ull) {
+        atomicMin(bad_arc, bad);
+    }
+    if (lo != ~0ull) {
+        atomicMin(min_len_bits, lo);
+    }
+    if (hi != 0ull) {
+        atomicMax(max_len_bits, hi);
+    }
+}
+
+// New lengths of the stored arcs, both metrics, from weights that passed the check.
+__global__ void update_lengths_kernel(const double* __restrict__ w, const int32_t* __restrict__ stored_of_user, int64_t m_user,
+                                      Arc* __restrict__ regular, Arc* __restrict__ inverse) {
+    for (int64_t e = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; e < m_user; e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+        const int32_t at = stored_of_user[e];
+        if (at >= 0) {
+            const double a = fabs(w[e]);
+            regular[at].len = a;
+            inverse[at].len = 1.0 / a;
+        }
+    }
+}
+
+// The in-arcs' lengths again, from the forward arcs they mirror.
+__global__ void update_reverse_kernel(const Arc* __restrict__ regular, int64_t m, Arc* __restrict__ rarcs) {
+    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < m; i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+        rarcs[i].len = regular[rarcs[i].id].len;
+    }
+}
+
 int grid_for(int64_t items, int per_block, int sm_count) {
     const int64_t want = (items + per_block - 1) / per_block;
     return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(want, static_cast<int64_t>(sm_count) * 16)));
@@ -302,6 +348,109 @@ int build_graph_on_device(const ngx_csr* csr, ngx_graph* g) {
     g->m_user = m_user;
     g->m_stored = m;
     g->max_out_degree = static_cast<int64_t>(red[1]);
+    return NGX_OK;
+}
+
+// In-place weight updates run on the device: the weights go up once (8 bytes per arc) and two passes of about 60 bytes per
+// arc rewrite the lengths, bound by memory bandwidth. Rewriting the three record arrays on the host and copying them both
+// ways took 41 of the 50 ms of an update of 2e6 arcs. Nothing changes when an arc is refused.
+int update_weights_on_device(ngx_graph* g, const double* w) {
+    const int64_t m_user = g->m_user;
+    if (m_user == 0) {
+        return NGX_OK;
+    }
+    cudaStream_t s = g->stream;
+    if (g->d_stored_of_user == nullptr) {
+        // a host-built handle keeps the map on the host: upload it once
+        NGX_CUDA_TRY(cudaMalloc(&g->d_stored_of_user, static_cast<size_t>(m_user) * 4));
+        NGX_CUDA_TRY(cudaMemcpyAsync(g->d_stored_of_user, g->stored_of_user.data(), static_cast<size_t>(m_user) * 4, cudaMemcpyHostToDevice, s));
+    }
+    // the weights and the check's results in the handle's call buffer (a run that follows reuses it in stream order)
+    if (const int rc = grow_buffer(g, &g->d_call_out, &g->call_out_bytes, 32 + static_cast<size_t>(m_user) * 8); rc != NGX_OK) {
+        return rc;
+    }
+    auto* d_red = static_cast<unsigned long long*>(g->d_call_out);  // bad arc, min length bits, max length bits
+    auto* d_w = reinterpret_cast<double*>(d_red + 4);
+    // the mean lengths, summed in stored order as the build sums them, beside the device work
+    struct Sums {
+        double regular = 0.0, inverse = 0.0;
+    };
+    std::vector<Sums> sums(g->parts.size() + 1);  // per graph, and over all graphs
+    const auto mean_sums = [&] {
+        Sums& all = sums.back();
+        const bool one = g->parts.size() == 1;  // the graph's sums are the handle's
+        for (size_t i = 0; i < g->parts.size(); ++i) {
+            const GraphPart& part = g->parts[i];
+            Sums own;
+            for (int64_t e = part.user_arc_off; e < part.user_arc_off + part.m_user; ++e) {
+                const double a = std::fabs(w[e]);
+                if (a == 0.0 || !std::isfinite(a)) {
+                    continue;
+                }
+                const double inv = 1.0 / a;
+                own.regular += a;
+                own.inverse += inv;
+                if (!one) {
+                    all.regular += a;
+                    all.inverse += inv;
+                }
+            }
+            sums[i] = own;
+            if (one) {
+                all = own;
+            }
+        }
+    };
+    std::thread sums_thread;
+    try {
+        sums_thread = std::thread(mean_sums);
+    } catch (const std::system_error&) {
+        mean_sums();  // no thread: summed here before the device work
+    }
+    struct Joiner {
+        std::thread& t;
+        ~Joiner() {
+            if (t.joinable()) {
+                t.join();
+            }
+        }
+    } joiner{ sums_thread };
+
+    unsigned long long red[4] = { ~0ull, ~0ull, 0ull, 0ull };
+    NGX_CUDA_TRY(cudaMemcpyAsync(d_red, red, sizeof(red), cudaMemcpyHostToDevice, s));
+    NGX_CUDA_TRY(cudaMemcpyAsync(d_w, w, static_cast<size_t>(m_user) * 8, cudaMemcpyHostToDevice, s));
+    const int grid = grid_for(m_user, kBuildBlock, g->sm_count);
+    check_weights_kernel<<<grid, kBuildBlock, 0, s>>>(d_w, g->d_stored_of_user, m_user, d_red, d_red + 1, d_red + 2);
+    NGX_CUDA_TRY(cudaGetLastError());
+    NGX_CUDA_TRY(cudaMemcpyAsync(red, d_red, sizeof(red), cudaMemcpyDeviceToHost, s));
+    NGX_CUDA_TRY(cudaStreamSynchronize(s));
+    if (red[0] != ~0ull) {
+        return fail(NGX_INVALID_ARGUMENT, "ngx_graph_update_weights: arc " + std::to_string(red[0]) +
+                                              " is non-finite or changes between zero and non-zero");
+    }
+    update_lengths_kernel<<<grid, kBuildBlock, 0, s>>>(d_w, g->d_stored_of_user, m_user, g->d_arcs_regular, g->d_arcs_inverse);
+    NGX_CUDA_TRY(cudaGetLastError());
+    if (g->m_stored > 0) {
+        update_reverse_kernel<<<grid_for(g->m_stored, kBuildBlock, g->sm_count), kBuildBlock, 0, s>>>(g->d_arcs_regular, g->m_stored, g->d_rarcs);
+        NGX_CUDA_TRY(cudaGetLastError());
+    }
+    NGX_CUDA_TRY(cudaStreamSynchronize(s));
+    if (sums_thread.joinable()) {
+        sums_thread.join();
+    }
+    for (size_t i = 0; i < g->parts.size(); ++i) {
+        GraphPart& part = g->parts[i];
+        if (part.m_stored > 0) {
+            part.mean_len_regular = sums[i].regular / static_cast<double>(part.m_stored);
+            part.mean_len_inverse = sums[i].inverse / static_cast<double>(part.m_stored);
+        }
+    }
+    if (g->m_stored > 0) {
+        g->mean_len_regular = sums.back().regular / static_cast<double>(g->m_stored);
+        g->mean_len_inverse = sums.back().inverse / static_cast<double>(g->m_stored);
+        std::memcpy(&g->min_len_regular, &red[1], 8);
+        std::memcpy(&g->max_len_regular, &red[2], 8);
+    }
     return NGX_OK;
 }
 

@@ -69,7 +69,7 @@ struct ngx_graph {
     int64_t* d_rrow_ptr = nullptr;
     ngx::Arc* d_rarcs = nullptr;
     int32_t* d_arc_src = nullptr;  // source vertex (graph-local) of each stored forward arc
-    int32_t* d_stored_of_user = nullptr;  // device build: stored index of each caller arc (-1 for zero weights)
+    int32_t* d_stored_of_user = nullptr;  // stored index of each caller arc (-1 for zero weights); host build: once needed
 
     double mean_len_regular = 1.0;
     double mean_len_inverse = 1.0;
@@ -106,8 +106,8 @@ struct ngx_graph {
     // launch shape and bucket width picked by ngx_graph_autotune, per task (APSP, Brandes, gradient); runs use them
     // for the options they leave at 0
     ngx_tuning tuned[3] = {};
-    // stored forward index of each caller arc (-1 for zero weights), for ngx_graph_update_weights (a device-built
-    // handle copies it from d_stored_of_user on first use)
+    // stored forward index of each caller arc (-1 for zero weights) of a host-built handle; ngx_graph_update_weights
+    // uploads it to d_stored_of_user on first use
     ngx::HostVector<int32_t> stored_of_user;
     // all-sources processing order of each graph (graph-local ids, graph after graph): clusters of nearby vertices,
     // so that the 32 sources of a tile reach most vertices in the same phases and share arc passes
@@ -165,8 +165,8 @@ int ensure_source_order(ngx_graph* g);
 // The strongly connected components of a single-graph handle (ngx_scc on its device), counted once per handle.
 int ensure_components(ngx_graph* g);
 
-// Copies a device-built handle's stored index of every caller arc to the host (ngx_graph_update_weights needs it).
-int ensure_stored_of_user(ngx_graph* g);
+// New weights for every caller arc of the handle (ngx_graph_update_weights), checked and written by device kernels.
+int update_weights_on_device(ngx_graph* g, const double* w);
 
 // Grows the graph's cached workspace to at least `bytes`.
 int ensure_workspace(ngx_graph* g, size_t bytes);
