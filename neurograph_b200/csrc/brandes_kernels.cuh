@@ -488,7 +488,7 @@ template <int kMode, bool kTree>
 __device__ __forceinline__ void dag_delta_level(const DeviceCsr& g, const int32_t* entries, int len, const unsigned long long* dist, const double* sigma,
                                                 double* delta, double* delta_g, const uint32_t* soff, const uint32_t* succ, unsigned long long* grad_cpl,
                                                 unsigned long long* grad_eff, double* buf, int lane, int buf_warp, int warp, int nwarps) {
-    constexpr bool kTarget = kMode == kModeBrandes;
+    constexpr bool kTarget = kMode == kModeBrandes || kTree;  // lists of targets: the arcs are not needed here
     constexpr int kU = delta_level_unroll(kMode);
     double* const wbuf = buf + static_cast<size_t>(buf_warp) * 32 * kU * (kMode == kModeGrad ? 2 : 1);
     for (int base = warp * 32; base < len; base += nwarps * 32) {
@@ -546,6 +546,10 @@ __device__ __forceinline__ void dag_delta_level(const DeviceCsr& g, const int32_
                 if (ok[u]) {
                     if constexpr (kMode == kModeBrandes) {
                         c = share_sv[u] * ((1.0 + dx[u]) / sx[u]);
+                    } else if constexpr (kTree) {
+                        const double inv = 1.0 / gx[u];  // every share is 1; the arcs get their terms in the epilogue
+                        c = 1.0 + dx[u];
+                        cg = inv * inv + dgx[u];
                     } else {
                         const double share = share_sv[u] / sx[u];
                         const double inv = 1.0 / gx[u];
@@ -578,6 +582,46 @@ __device__ __forceinline__ void dag_delta_level(const DeviceCsr& g, const int32_
             if constexpr (kMode == kModeGrad) {
                 delta_g[row] = acc_g;
             }
+        }
+    }
+}
+
+// Adds each active lane's terms c (a whole number) and cg to the gradients of its arc e, in 128-bit fixed point. The
+// sources of a tile are near one another, so most lanes of a vertex share its predecessor arc: the lanes of one arc are
+// summed first (exactly: integer adds), and one lane per arc adds the sums, a third of the atomics at out-degree 40.
+__device__ __forceinline__ void add_arc_terms(const Arc* arcs, bool active, uint32_t e, double c, double cg, int lane, unsigned long long* grad_cpl,
+                                              unsigned long long* grad_eff) {
+    const unsigned act = __ballot_sync(0xFFFFFFFFu, active);
+    if (!active) {
+        return;
+    }
+    unsigned long long sum = static_cast<unsigned long long>(c);
+    unsigned long long lo, hi;
+    fixed_parts(cg, lo, hi);
+    const unsigned all = __match_any_sync(act, e);
+    unsigned peers = all & (0xFFFFFFFEu << lane);  // the arc's lanes above this one
+    int rank = __popc(all & lanemask_lt());
+    while (__any_sync(act, peers != 0u)) {
+        const int next = __ffs(peers);
+        const int from = next != 0 ? next - 1 : lane;
+        const unsigned long long o_sum = __shfl_sync(act, sum, from);
+        const unsigned long long o_lo = __shfl_sync(act, lo, from);
+        const unsigned long long o_hi = __shfl_sync(act, hi, from);
+        if (next != 0) {
+            sum += o_sum;
+            const unsigned long long t = lo + o_lo;
+            hi += o_hi + (t < lo ? 1ull : 0ull);
+            lo = t;
+        }
+        // lanes of odd rank have been added to the one below and drop out
+        peers &= __ballot_sync(act, (rank & 1) == 0);
+        rank >>= 1;
+    }
+    if (lane == __ffs(all) - 1) {
+        const int64_t id = ldg_arc(&arcs[e]).id;
+        atomicAdd(&grad_cpl[2 * id + 1], sum);
+        if ((lo | hi) != 0ull) {
+            fixed_add_parts(&grad_eff[2 * id], lo, hi);
         }
     }
 }

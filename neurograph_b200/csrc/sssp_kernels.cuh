@@ -651,10 +651,11 @@ __device__ __forceinline__ void scan_in_arcs(const TileSmem& sh, WarpScratch& w,
 }
 
 // cnt[v][s] = DAG predecessors of (v, s), pred[v][s] = forward index of one of their arcs (the only one when cnt is 1),
-// scnt[u][s] += 1 for each DAG arc u -> v, sigma = 0; warp per vertex, lane per source. parent[v][s] (unless nullptr) =
-// that arc's source. src_lane: this lane's source vertex (-1 without one).
+// scnt[u][s] += 1 for each DAG arc u -> v, sigma = 0; warp per vertex, lane per source. keep[v][s] = that arc's
+// source (kKeepArc: its forward index), for passes after pred's storage is reused. src_lane: this lane's source vertex (-1 without one).
+template <bool kKeepArc>
 __device__ __noinline__ void dag_count(const uint32_t* low, int src_lane, double* sigma, uint32_t* cnt, uint32_t* scnt, uint32_t* pred,
-                                       uint32_t* parent, TileShared* ctl, int gw) {
+                                       uint32_t* keep, TileShared* ctl, int gw) {
     extern __shared__ __align__(16) unsigned long long smem[];
     TileSmem& sh = *reinterpret_cast<TileSmem*>(smem);
     const int lane = threadIdx.x & 31;
@@ -680,9 +681,7 @@ __device__ __noinline__ void dag_count(const uint32_t* low, int src_lane, double
         sigma[row] = 0.0;
         cnt[row] = c;
         pred[row] = first;
-        if (parent != nullptr) {
-            parent[row] = static_cast<uint32_t>(from);
-        }
+        keep[row] = kKeepArc ? first : static_cast<uint32_t>(from);
         arc_count += c;
     }
     const unsigned pairs = __reduce_add_sync(kFullMask, active_count);
@@ -1127,7 +1126,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
             atomicAdd(&cnts[kCyclesSssp], static_cast<unsigned long long>(now - t_phase));
             t_phase = now;
         }
-        bool tree_walk = false;
+        bool tree = false;
         if constexpr (kMode != kModeApsp) {
             // ------------------------------------------------------------ shortest-path DAG: counts, sigma, delta
             // the level lists are built only after the successor lists: their storage holds pred[][] until then
@@ -1135,9 +1134,12 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
             uint32_t* const low = stamp;  // its words held the distance phase's bounds until here
             dag_low(dist, low, n, nsrc, lane, NGX_GW, NGX_GWARPS);
             sync0();
-            dag_count(low, lane < nsrc ? s_src[lane] : -1, sigma, cnt, scnt, pred, kMode == kModeBrandes ? lvl : nullptr, ctl(), NGX_GW);
+            dag_count<kMode == kModeGrad>(low, lane < nsrc ? s_src[lane] : -1, sigma, cnt, scnt, pred, lvl, ctl(), NGX_GW);
             sync0();
-            tree_walk = kMode == kModeBrandes && s.dag_arcs == s.active_pairs && b.succ_capacity > 0;
+            // when every reached pair has exactly one DAG predecessor (as many DAG arcs as reached non-source pairs) the
+            // DAGs are trees
+            tree = s.dag_arcs == s.active_pairs && b.succ_capacity > 0;
+            const bool tree_walk = kMode == kModeBrandes && tree;
           if (tree_walk) {
             if (tid == 0) {
                 const long long now = clock64();
@@ -1162,7 +1164,11 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
             }
             sync0();
             if (use_lists) {
-                dag_fill<kMode == kModeBrandes>(b.arc_src, low, cnt, pred, soff, scnt, succ, NGX_GW);
+                if (kMode == kModeBrandes || tree) {
+                    dag_fill<true>(b.arc_src, low, cnt, pred, soff, scnt, succ, NGX_GW);
+                } else {
+                    dag_fill<false>(b.arc_src, low, cnt, pred, soff, scnt, succ, NGX_GW);
+                }
                 sync0();
                 dag_sort(soff, succ, nt, NGX_GT, NGX_GTHREADS);
             }
@@ -1210,10 +1216,8 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
             }
             sync0();
           if (use_lists) {
-            // --- sigma and delta over the successor lists. When every reached pair has exactly one DAG predecessor
-            // (as many DAG arcs as reached non-source pairs) the DAGs are trees: every sigma is 1 and every child is
-            // released by its only parent, so the sigma levels need neither sums nor counts.
-            const bool tree = dag_arcs == s.active_pairs;
+            // --- sigma and delta over the successor lists. In a tree every sigma is 1 and every child is released by its
+            // only parent, so the sigma levels need neither sums nor counts.
             for (;;) {
                 const int start = s.lvl_start;
                 const int len = s.lvl_len;
@@ -1222,7 +1226,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
                 }
                 const unsigned level = s.level;
                 if (tree) {
-                    dag_tree_level<kMode == kModeBrandes>(g, list + start, len, sigma, soff, succ, list + start + len, &ctl()->next_len, lane, NGX_GW,
+                    dag_tree_level<true>(g, list + start, len, sigma, soff, succ, list + start + len, &ctl()->next_len, lane, NGX_GW,
                                                           NGX_GWARPS);
                 } else {
                     dag_sigma_level<kMode == kModeBrandes>(g, list + start, len, sigma, cnt, soff, succ, list + start + len, &ctl()->next_len,
@@ -1242,7 +1246,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
                 t_phase = now;
             }
             const int levels = static_cast<int>(s.level);
-            const int lowest = kMode == kModeGrad ? 0 : 1;
+            const int lowest = kMode == kModeGrad && !tree ? 0 : 1;  // the sources' own arcs get their terms from level 0, in a tree in the epilogue
             for (int level = levels - 1; level >= lowest; --level) {
                 const int start = __ldcg(&loff[level]);
                 const int end = __ldcg(&loff[level + 1]);
@@ -1361,7 +1365,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
                 if constexpr (kMode == kModeBrandes) {
                     // BrandesVariant.h:156: every settled vertex but the source gains its dependency
                     const bool gains = valid && v != my_src && bits != kInfBits;
-                    if (tree_walk) {
+                    if (tree) {
                         // integers (descendant counts): exact in double and in fixed point alike
                         const unsigned long long dep = gains ? __ldcg(reinterpret_cast<unsigned long long*>(&sigma[row])) & 0xFFFFFFFFull : 0ull;
                         const unsigned long long sum = __reduce_add_sync(kFullMask, static_cast<unsigned>(dep & 0xFFFFull)) +
@@ -1380,6 +1384,11 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
                             fixed_add_parts(&bc_g[2 * v], lo, hi);
                         }
                     }
+                } else if (tree) {
+                    const bool on = valid && v != my_src && bits != kInfBits;
+                    const double inv = on ? 1.0 / __longlong_as_double(static_cast<long long>(bits)) : 0.0;
+                    add_arc_terms(g.arcs, on, on ? __ldcg(&lvl[row]) : 0u, on ? 1.0 + __ldcg(&delta[row]) : 0.0,
+                                  on ? inv * inv + __ldcg(&delta_g[row]) : 0.0, lane, b.grad_cpl, b.grad_eff);
                 }
                 scnt[row] = 0u;
             }
