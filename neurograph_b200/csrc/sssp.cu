@@ -184,18 +184,21 @@ const void* tile_kernel_for_block(int block, int ctas_per_sm, bool reach, bool m
     }
 }
 
-// CTAs per tile group: the caller's choice, else by the sizes of the job's graphs and its number of tiles.
+// CTAs per tile group: the caller's choice, else the size with the least modelled time.
 //  * Work per phase. A tile's phases (near iterations, bucket steps, DAG passes) end with a barrier of its group, and the
-//    entries of a phase grow with n while their number grows slowly, so larger graphs feed more CTAs: about
-//    0.12 sqrt(n), as many tiles in flight as then fit in the resident CTAs, at least four. Measured kernel times
-//    (Brandes unless noted, CTAs per tile: ms): n = 1e4, degree 40: 3: 79, 7: 62, 10-14: 58, 24: 66; n = 2e4, degree 6:
-//    1: 267, 4: 217, 14: 197; n = 3e4, degree 40: 7: 183, 21: 152, 42: 156; n = 5e4 (gradient): 9: 73, 18-37: 67, 49: 69;
-//    n = 1e5, degree 100 (APSP): 37-49: 176, 74: 179, 148: 234; n = 3e5, degree 40: 4: 337, 37-74: 264, 100: 325;
-//    n = 1e6: 18: 309, 74: 279; batches of mixed graphs, mean n 800: 1: 19.3, 2: 16.4, 8: 29; 3200: 1: 138, 6: 127, 11: 156;
-//    13,400: 1: 637, 11: 522, 24: 581. Keeping the tiles in flight within L2 matters less: the rate of random sector
-//    reads halves between 65 and 100 MB (microbenchmark), but the barriers of larger groups cost more than that.
-//  * Few tiles: a run with fewer tiles than resident CTAs gives each tile the CTAs the others would leave idle, up to five
-//    times the above (n = 2e4, 2 tiles: 37: 1.22, 74: 0.94, 148: 1.05 ms; n = 300, 10 tiles: 4: 0.49, 8-16: 0.45).
+//    entries of a phase grow with n while their number grows slowly, so larger graphs feed more CTAs. Measured kernel
+//    times over many tiles (Brandes unless noted, CTAs per tile: ms): n = 1e4, degree 40: 3: 79, 7: 62, 10-14: 58, 24: 66;
+//    n = 2e4, degree 6: 1: 267, 4: 217, 14: 197; n = 3e4, degree 40: 7: 183, 21: 152, 42: 156; n = 5e4 (gradient): 9: 73,
+//    18-37: 67, 49: 69; n = 1e5, degree 100 (APSP): 37-49: 176, 74: 179, 148: 234; n = 3e5, degree 40: 4: 337, 37-74: 264,
+//    100: 325; n = 1e6: 18: 309, 74: 279; batches of mixed graphs, mean n 800: 1: 19.3, 2: 16.4, 8: 29; 3200: 1: 138, 6: 127,
+//    11: 156; 13,400: 1: 637, 11: 522, 24: 581. Those follow (1 + b + l) / g for a tile's time: b = 250 g / n (1 + g / 100)
+//    for the barriers, more by the cube root of the degree below 40 (less work per phase), and l = 0.2 for each doubling of
+//    the distance-phase bytes in flight (280 per vertex and slot) beyond 65 MB, where the rate of random sector reads from
+//    L2 starts to fall (microbenchmark: half at 100 MB).
+//  * Waves. The tiles run in waves of resident / g, counted whole when there are few: 63 tiles of n = 2000 (gradient) want
+//    4 CTAs and one wave (2.2 ms; 3: 2.6, 5 and two waves: 3.1, 9: 2.7). Few tiles take the CTAs that would idle, up to
+//    0.6 sqrt(n) (n = 2e4, 2 tiles: 37: 1.22, 74: 0.94, 148: 1.05 ms; n = 300, 10 tiles: 4: 0.49, 8-29: 0.45). At least
+//    four tiles stay in flight.
 //  * Sparse graphs (mean out-degree below 4) have long shortest paths, so many phases with few entries each: one CTA per
 //    tile while there are two tiles for every resident CTA (n = 2e4, degree 2, 626 tiles: 1: 70, 3: 75, 7: 92, 14: 118 ms),
 //    more in proportion when there are fewer.
@@ -204,15 +207,29 @@ int choose_group_size(int requested, int64_t resident, int64_t num_tiles, int64_
     if (requested > 0) {
         return static_cast<int>(std::min<int64_t>({ static_cast<int64_t>(requested), resident, static_cast<int64_t>(kMaxGroupSize) }));
     }
-    const double wanted = 0.12 * std::sqrt(std::max(typical_n, 1.0));
-    int64_t in_flight = static_cast<int64_t>(static_cast<double>(resident) / std::max(wanted, 1.0) + 0.5);
-    in_flight = std::max<int64_t>(in_flight, 4);
-    int64_t group = std::max<int64_t>(1, resident / in_flight);
+    const int64_t tiles = std::max<int64_t>(1, num_tiles);
+    const double n = std::max(typical_n, 1.0);
+    const double sparse = std::cbrt(std::max(1.0, 40.0 / std::max(mean_degree, 1.0)));
+    int64_t most = std::min(std::max(resident / 4, resident / tiles), static_cast<int64_t>(0.6 * std::sqrt(n)));
     if (mean_degree < 4.0) {
-        group = std::min(group, std::max<int64_t>(1, 2 * resident / std::max<int64_t>(1, num_tiles)));
+        most = std::min(most, std::max<int64_t>(1, 2 * resident / tiles));
     }
-    const int64_t idle_share = resident / std::max<int64_t>(1, num_tiles);
-    group = std::max(group, std::min(idle_share, static_cast<int64_t>(5.0 * wanted)));
+    most = std::max<int64_t>(1, std::min({ most, resident, static_cast<int64_t>(kMaxGroupSize) }));
+    int64_t group = 1;
+    double least = INFINITY;
+    for (int64_t g = 1; g <= most; ++g) {
+        const int64_t slots = resident / g;
+        const double waves = tiles > 8 * slots ? static_cast<double>(tiles) / static_cast<double>(slots)
+                                               : static_cast<double>((tiles + slots - 1) / slots);
+        const double size = static_cast<double>(g);
+        const double in_flight = 280.0 * n * static_cast<double>(std::min(slots, tiles));
+        const double barriers = 250.0 * sparse * size / n * (1.0 + size / 100.0);
+        const double time = waves * (1.0 + barriers + 0.2 * std::max(0.0, std::log2(in_flight / 65e6))) / size;
+        if (time < least) {
+            least = time;
+            group = g;
+        }
+    }
     if (affordable_slots < std::min(resident, num_tiles)) {
         // enough CTAs per slot that the affordable slots hold every resident CTA (rounded up: the slot count then
         // follows from the group size, and no CTA is left without a slot)
