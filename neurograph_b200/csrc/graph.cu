@@ -167,13 +167,23 @@ void release(ngx_graph* g) {
     if (g->stream != nullptr) {
         cudaStreamSynchronize(g->stream);
     }
-    cudaFree(g->d_row_ptr);
-    cudaFree(g->d_arcs_regular);
-    cudaFree(g->d_arcs_inverse);
-    cudaFree(g->d_rrow_ptr);
-    cudaFree(g->d_rarcs);
-    cudaFree(g->d_arc_src);
-    cudaFree(g->d_stored_of_user);
+    if (g->d_block != nullptr) {
+        cudaFree(g->d_block);
+    } else {
+        cudaFree(g->d_row_ptr);
+        cudaFree(g->d_arcs_regular);
+        cudaFree(g->d_arcs_inverse);
+        cudaFree(g->d_rrow_ptr);
+        cudaFree(g->d_rarcs);
+        cudaFree(g->d_arc_src);
+        cudaFree(g->d_stored_of_user);
+    }
+    if (g->run_start != nullptr) {
+        cudaEventDestroy(g->run_start);
+    }
+    if (g->run_stop != nullptr) {
+        cudaEventDestroy(g->run_stop);
+    }
     cudaFree(g->d_workspace);
     cudaFree(g->d_items);
     cudaFree(g->d_persistent);
@@ -574,9 +584,13 @@ int create_graphs(const ngx_csr* csrs, int64_t count, int device, ngx_graph** ou
         return fail(NGX_INVALID_ARGUMENT, "ngx_graph_create: no CUDA device " + std::to_string(device));
     }
     NGX_CUDA_TRY(cudaSetDevice(device));
-    cudaDeviceProp prop{};
-    NGX_CUDA_TRY(cudaGetDeviceProperties(&prop, device));
-    if (prop.major != 10) {
+    // two attributes instead of all properties, which take the driver about a millisecond
+    int major = 0, sm_count = 0;
+    NGX_CUDA_TRY(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device));
+    NGX_CUDA_TRY(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device));
+    if (major != 10) {
+        cudaDeviceProp prop{};
+        NGX_CUDA_TRY(cudaGetDeviceProperties(&prop, device));
         return fail(NGX_UNSUPPORTED, std::string("ngx_graph_create: the kernels are built for sm_100a (B200); device is ") + prop.name);
     }
 
@@ -585,7 +599,7 @@ int create_graphs(const ngx_csr* csrs, int64_t count, int device, ngx_graph** ou
         return fail(NGX_OUT_OF_MEMORY, "ngx_graph_create: host allocation failed");
     }
     g->device = device;
-    g->sm_count = prop.multiProcessorCount;
+    g->sm_count = sm_count;
     if (!on_device) {
         g->n_total = h.n_total;
         g->m_user = h.m_user;

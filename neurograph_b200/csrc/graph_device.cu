@@ -185,23 +185,33 @@ int bits_for(int64_t n) {
     return b;
 }
 
-// Temporary device buffers of the build, freed on every exit.
-struct Scratch {
-    void* p[12] = {};
-    int used = 0;
-    ~Scratch() {
-        for (int i = 0; i < used; ++i) {
-            cudaFree(p[i]);
-        }
-    }
+// Arrays carved from one allocation (cudaMalloc and cudaFree take tens of microseconds each, more than the kernels of a
+// small build): first every array is announced, then the block is allocated and the pointers are set.
+struct Carver {
+    struct Slot {
+        void** out;
+        size_t at;
+    };
+    std::vector<Slot> slots;
+    size_t bytes = 0;
     template <typename T>
-    int take(T** out, size_t count) {
-        void* ptr = nullptr;
-        NGX_CUDA_TRY(cudaMalloc(&ptr, std::max<size_t>(1, count) * sizeof(T)));
-        p[used++] = ptr;
-        *out = static_cast<T*>(ptr);
+    void take(T** out, size_t count) {
+        slots.push_back(Slot{ reinterpret_cast<void**>(out), bytes });
+        bytes += (std::max<size_t>(1, count) * sizeof(T) + 255) & ~size_t(255);
+    }
+    int allocate(void** block) const {
+        NGX_CUDA_TRY(cudaMalloc(block, bytes));
+        for (const Slot& s : slots) {
+            *s.out = static_cast<char*>(*block) + s.at;
+        }
         return NGX_OK;
     }
+};
+
+// The build's temporary block, freed on every exit.
+struct TempBlock {
+    void* p = nullptr;
+    ~TempBlock() { cudaFree(p); }
 };
 
 }  // namespace
@@ -239,18 +249,35 @@ int build_graph_on_device(const ngx_csr* csr, ngx_graph* g) {
         }
     } joiner{ sums_thread };
 
-    Scratch tmp;
+    // every array's size is known up front (no more arcs are stored than given)
+    const size_t mu = static_cast<size_t>(m_user);
     int64_t* d_user_rows = nullptr;
     int32_t* d_col = nullptr;
     double* d_w = nullptr;
     int64_t* d_kept = nullptr;
     unsigned long long* d_red = nullptr;  // bad arc, max degree, min length bits, max length bits
-    int rc = NGX_OK;
-    if ((rc = tmp.take(&d_user_rows, static_cast<size_t>(n) + 1)) != NGX_OK) return rc;
-    if ((rc = tmp.take(&d_col, static_cast<size_t>(m_user))) != NGX_OK) return rc;
-    if ((rc = tmp.take(&d_w, static_cast<size_t>(m_user))) != NGX_OK) return rc;
-    if ((rc = tmp.take(&d_kept, static_cast<size_t>(n) + 1)) != NGX_OK) return rc;
-    if ((rc = tmp.take(&d_red, 4)) != NGX_OK) return rc;
+    uint32_t *d_target = nullptr, *d_target_sorted = nullptr;  // unsigned keys: the sort looks at the low bits only
+    int32_t *d_index = nullptr, *d_index_sorted = nullptr;
+    char *d_scan = nullptr, *d_sort = nullptr;
+    size_t scan_bytes = 0, sort_bytes = 0;
+    NGX_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, d_kept, g->d_row_ptr, n + 1, s));
+    NGX_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, d_target, d_target_sorted, d_index, d_index_sorted, m_user, 0, bits_for(n), s));
+    TempBlock tmp;
+    Carver temps;
+    temps.take(&d_user_rows, static_cast<size_t>(n) + 1);
+    temps.take(&d_col, mu);
+    temps.take(&d_w, mu);
+    temps.take(&d_kept, static_cast<size_t>(n) + 1);
+    temps.take(&d_red, 4);
+    temps.take(&d_target, mu);
+    temps.take(&d_index, mu);
+    temps.take(&d_target_sorted, mu);
+    temps.take(&d_index_sorted, mu);
+    temps.take(&d_scan, scan_bytes);
+    temps.take(&d_sort, sort_bytes);
+    if (const int rc = temps.allocate(&tmp.p); rc != NGX_OK) {
+        return rc;
+    }
     NGX_CUDA_TRY(cudaMemcpyAsync(d_user_rows, csr->row_ptr, (static_cast<size_t>(n) + 1) * 8, cudaMemcpyHostToDevice, s));
     if (m_user > 0) {
         NGX_CUDA_TRY(cudaMemcpyAsync(d_col, csr->col, static_cast<size_t>(m_user) * 4, cudaMemcpyHostToDevice, s));
@@ -272,28 +299,23 @@ int build_graph_on_device(const ngx_csr* csr, ngx_graph* g) {
                                               (bad_target ? " has an out-of-range target" : " has a non-finite weight"));
     }
 
+    Carver arrays;
+    arrays.take(&g->d_row_ptr, static_cast<size_t>(n) + 1);
+    arrays.take(&g->d_rrow_ptr, static_cast<size_t>(n) + 1);
+    arrays.take(&g->d_arcs_regular, mu);
+    arrays.take(&g->d_arcs_inverse, mu);
+    arrays.take(&g->d_rarcs, mu);
+    arrays.take(&g->d_arc_src, mu);
+    arrays.take(&g->d_stored_of_user, mu);
+    if (const int rc = arrays.allocate(&g->d_block); rc != NGX_OK) {
+        return rc;
+    }
     // stored row offsets: exclusive sum of the kept counts (n + 1 entries, the last one m)
-    NGX_CUDA_TRY(cudaMalloc(&g->d_row_ptr, (static_cast<size_t>(n) + 1) * 8));
-    size_t scan_bytes = 0;
-    NGX_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, d_kept, g->d_row_ptr, n + 1, s));
-    char* d_scan = nullptr;
-    if ((rc = tmp.take(&d_scan, scan_bytes)) != NGX_OK) return rc;
     NGX_CUDA_TRY(cub::DeviceScan::ExclusiveSum(d_scan, scan_bytes, d_kept, g->d_row_ptr, n + 1, s));
     int64_t m = 0;
     NGX_CUDA_TRY(cudaMemcpyAsync(&m, g->d_row_ptr + n, 8, cudaMemcpyDeviceToHost, s));
     NGX_CUDA_TRY(cudaStreamSynchronize(s));
 
-    const size_t ms = static_cast<size_t>(m);
-    NGX_CUDA_TRY(cudaMalloc(&g->d_arcs_regular, std::max<size_t>(1, ms) * sizeof(Arc)));
-    NGX_CUDA_TRY(cudaMalloc(&g->d_arcs_inverse, std::max<size_t>(1, ms) * sizeof(Arc)));
-    NGX_CUDA_TRY(cudaMalloc(&g->d_arc_src, std::max<size_t>(1, ms) * 4));
-    NGX_CUDA_TRY(cudaMalloc(&g->d_stored_of_user, std::max<int64_t>(1, m_user) * 4));
-    uint32_t *d_target = nullptr, *d_target_sorted = nullptr;  // unsigned keys: the sort looks at the low bits only
-    int32_t *d_index = nullptr, *d_index_sorted = nullptr;
-    if ((rc = tmp.take(&d_target, ms)) != NGX_OK) return rc;
-    if ((rc = tmp.take(&d_index, ms)) != NGX_OK) return rc;
-    if ((rc = tmp.take(&d_target_sorted, ms)) != NGX_OK) return rc;
-    if ((rc = tmp.take(&d_index_sorted, ms)) != NGX_OK) return rc;
     fill_rows_kernel<<<row_grid, kBuildBlock, 0, s>>>(d_user_rows, d_col, d_w, n, g->d_row_ptr, g->d_arcs_regular, g->d_arcs_inverse, g->d_arc_src,
                                                       g->d_stored_of_user, d_target, d_index);
     NGX_CUDA_TRY(cudaGetLastError());
@@ -305,14 +327,19 @@ int build_graph_on_device(const ngx_csr* csr, ngx_graph* g) {
         in_degree_kernel<<<grid_for(m, kBuildBlock, g->sm_count), kBuildBlock, 0, s>>>(d_target, m, d_kept);
         NGX_CUDA_TRY(cudaGetLastError());
     }
-    NGX_CUDA_TRY(cudaMalloc(&g->d_rrow_ptr, (static_cast<size_t>(n) + 1) * 8));
     NGX_CUDA_TRY(cub::DeviceScan::ExclusiveSum(d_scan, scan_bytes, d_kept, g->d_rrow_ptr, n + 1, s));
-    NGX_CUDA_TRY(cudaMalloc(&g->d_rarcs, std::max<size_t>(1, ms) * sizeof(Arc)));
     if (m > 0) {
-        size_t sort_bytes = 0;
-        NGX_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, d_target, d_target_sorted, d_index, d_index_sorted, m, 0, bits_for(n), s));
-        char* d_sort = nullptr;
-        if ((rc = tmp.take(&d_sort, sort_bytes)) != NGX_OK) return rc;
+        // the temporary storage was sized for m_user pairs; fewer (zero weights dropped) should need no more
+        TempBlock more;
+        if (m != m_user) {
+            size_t need = 0;
+            NGX_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, need, d_target, d_target_sorted, d_index, d_index_sorted, m, 0, bits_for(n), s));
+            if (need > sort_bytes) {
+                NGX_CUDA_TRY(cudaMalloc(&more.p, need));
+                d_sort = static_cast<char*>(more.p);
+                sort_bytes = need;
+            }
+        }
         NGX_CUDA_TRY(cub::DeviceRadixSort::SortPairs(d_sort, sort_bytes, d_target, d_target_sorted, d_index, d_index_sorted, m, 0, bits_for(n), s));
         reverse_records_kernel<<<grid_for(m, kBuildBlock, g->sm_count), kBuildBlock, 0, s>>>(d_index_sorted, m, g->d_arcs_regular, g->d_arc_src,
                                                                                             g->d_rarcs);

@@ -61,6 +61,8 @@ struct ngx_graph {
     void* d_items = nullptr;
     int64_t num_items = 0;
 
+    // One allocation for all arrays of a device-built graph (nullptr: they are separate allocations).
+    void* d_block = nullptr;
     // Forward CSR over stored arcs; two arc arrays, one per metric (|w| and 1/|w|).
     int64_t* d_row_ptr = nullptr;
     ngx::Arc* d_arcs_regular = nullptr;
@@ -82,6 +84,10 @@ struct ngx_graph {
     int* d_abort = nullptr;
 
     uint64_t memory_budget = 0;
+
+    // events around the tile kernel of synchronous runs, created with the first
+    cudaEvent_t run_start = nullptr;
+    cudaEvent_t run_stop = nullptr;
 
     // Cached device workspace, grown on demand and reused across runs.
     void* d_workspace = nullptr;

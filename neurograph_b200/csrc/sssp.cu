@@ -10,6 +10,7 @@
 #include <cmath>
 #include <cstring>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "ngx_common.cuh"
@@ -304,21 +305,30 @@ int launch_tiles(ngx_graph* g, const ngx_apsp_opts* opts, int tile_mode, const T
     const size_t reach_bytes = track ? static_cast<size_t>(n) * 8 + 512 : 0;  // reach mask + reached list
     const size_t dag_bytes = tile_mode == kModeApsp ? 0 : batched ? brandes_slot_bytes(n, tile_mode == kModeGrad) : plain_brandes_slot_bytes(n);
     const size_t data_bytes = sssp_slot_bytes(n, width) + dag_bytes + reach_bytes;
-    const size_t budget = workspace_budget(g);
     // the sizes the group rule goes by: the graph's, or the mean over a batch's graphs
     const double typical_n = job.num_graphs > 1 ? static_cast<double>(g->n_total) / static_cast<double>(job.num_graphs) : static_cast<double>(n);
     const double mean_degree = static_cast<double>(job.num_arcs) / std::max(1.0, typical_n * static_cast<double>(job.num_graphs));
-    // the group size decides the group storage per slot, which the slot count must leave room for
-    const int64_t affordable = static_cast<int64_t>(budget / (data_bytes + static_cast<size_t>(group_stride_words(kMaxGroupSize)) * 8));
-    const int group = batched && default_shape ? choose_group_size(opts->tile_ctas, resident, num_tiles, affordable, typical_n, mean_degree) : 1;
+    const auto group_bytes_of = [](int ctas) { return static_cast<size_t>(group_stride_words(ctas)) * 8; };
+    const auto slots_of = [&](int ctas) { return std::min<int64_t>(num_tiles, resident / ctas); };
+    // a workspace kept from an earlier run that holds what an unlimited device would get needs no look at the free memory
+    // (a driver call of tens of microseconds)
+    int group = batched && default_shape ? choose_group_size(opts->tile_ctas, resident, num_tiles, resident, typical_n, mean_degree) : 1;
+    size_t slot_bytes = data_bytes + group_bytes_of(group);
+    int64_t slots = slots_of(group);
+    const size_t kept = g->memory_budget != 0 ? std::min<size_t>(g->workspace_bytes, static_cast<size_t>(g->memory_budget)) : g->workspace_bytes;
+    if (static_cast<size_t>(slots) * slot_bytes > kept) {
+        const size_t budget = workspace_budget(g);
+        // the group size decides the group storage per slot, which the slot count must leave room for
+        const int64_t affordable = static_cast<int64_t>(budget / (data_bytes + group_bytes_of(kMaxGroupSize)));
+        group = batched && default_shape ? choose_group_size(opts->tile_ctas, resident, num_tiles, affordable, typical_n, mean_degree) : 1;
+        slot_bytes = data_bytes + group_bytes_of(group);
+        slots = std::min<int64_t>(slots_of(group), static_cast<int64_t>(budget / slot_bytes));
+    }
     if (group > 1) {
         kernel = pick(track, true);  // the same shape and occupancy, built for groups
         NGX_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     }
-    const size_t group_bytes = static_cast<size_t>(group_stride_words(group)) * 8;
-    const size_t slot_bytes = data_bytes + group_bytes;
-    int64_t slots = std::min<int64_t>(num_tiles, resident / group);
-    slots = std::min<int64_t>(slots, static_cast<int64_t>(budget / slot_bytes));
+    const size_t group_bytes = group_bytes_of(group);
     if (slots <= 0) {
         return fail(NGX_OUT_OF_MEMORY, "not enough device memory for one workspace slot (" + std::to_string(slot_bytes) + " bytes)");
     }
@@ -428,11 +438,14 @@ int launch_tiles(ngx_graph* g, const ngx_apsp_opts* opts, int tile_mode, const T
     p.out.src_arcs = o.src_u64 + job.num_sources;
     p.out.rows = o.rows;
 
-    cudaEvent_t start = nullptr, stop = nullptr;
     if (synchronous) {
-        NGX_CUDA_TRY(cudaEventCreate(&start));
-        NGX_CUDA_TRY(cudaEventCreate(&stop));
-        cudaEventRecord(start, g->stream);
+        if (g->run_start == nullptr) {
+            NGX_CUDA_TRY(cudaEventCreate(&g->run_start));
+        }
+        if (g->run_stop == nullptr) {
+            NGX_CUDA_TRY(cudaEventCreate(&g->run_stop));
+        }
+        cudaEventRecord(g->run_start, g->stream);
     }
     cudaError_t err = cudaSuccess;
     if (batched) {
@@ -452,24 +465,23 @@ int launch_tiles(ngx_graph* g, const ngx_apsp_opts* opts, int tile_mode, const T
     if (!synchronous) {
         return err == cudaSuccess ? NGX_OK : cuda_fail(err, "tile kernel launch");
     }
-    cudaEventRecord(stop, g->stream);
+    cudaEventRecord(g->run_stop, g->stream);
+    int code = 0;
     if (err == cudaSuccess) {
-        err = cudaEventSynchronize(stop);
+        err = cudaMemcpyAsync(&code, o.error, sizeof(int), cudaMemcpyDeviceToHost, g->stream);
     }
+    const cudaError_t done = cudaStreamSynchronize(g->stream);
+    err = err == cudaSuccess ? done : err;
     float ms = 0.0f;
     if (err == cudaSuccess) {
-        cudaEventElapsedTime(&ms, start, stop);
+        err = cudaEventElapsedTime(&ms, g->run_start, g->run_stop);
     }
-    cudaEventDestroy(start);
-    cudaEventDestroy(stop);
     if (err != cudaSuccess) {
         return cuda_fail(err, "tile kernel");
     }
     if (kernel_ms != nullptr) {
         *kernel_ms += ms;
     }
-    int code = 0;
-    NGX_CUDA_TRY(cudaMemcpy(&code, o.error, sizeof(int), cudaMemcpyDeviceToHost));
     return device_error_status(code);
 }
 
@@ -606,25 +618,27 @@ int collect_graph(ngx_graph* g, const RunOutputs& o, const unsigned long long* a
     }
     if (s > 0 && scatter != nullptr) {
         // the run took the sources in the graph's locality order: entry i belongs to vertex scatter[i]
-        std::vector<unsigned long long> tmp(s);
-        const auto put = [&](void* dst, const void* src) -> int {
-            if (dst == nullptr) {
-                return NGX_OK;
+        // (all the wanted arrays come back with one wait)
+        const std::pair<void*, const void*> wanted[] = { { r->src_sum, o.src_f64 + at },
+                                                         { r->src_max, o.src_f64 + total + at },
+                                                         { r->src_sum_inverse, o.src_f64 + 2 * total + at },
+                                                         { r->src_unreachable, o.src_u64 + at },
+                                                         { r->src_arcs, o.src_u64 + total + at } };
+        std::vector<unsigned long long> tmp(5 * s);
+        for (size_t k = 0; k < 5; ++k) {
+            if (wanted[k].first != nullptr) {
+                NGX_CUDA_TRY(cudaMemcpyAsync(tmp.data() + k * s, wanted[k].second, s * 8, cudaMemcpyDeviceToHost, g->stream));
             }
-            NGX_CUDA_TRY(cudaMemcpyAsync(tmp.data(), src, s * 8, cudaMemcpyDeviceToHost, g->stream));
-            NGX_CUDA_TRY(cudaStreamSynchronize(g->stream));
-            auto* out = static_cast<unsigned long long*>(dst);
-            for (size_t i = 0; i < s; ++i) {
-                out[scatter[i]] = tmp[i];
+        }
+        NGX_CUDA_TRY(cudaStreamSynchronize(g->stream));
+        for (size_t k = 0; k < 5; ++k) {
+            if (auto* out = static_cast<unsigned long long*>(wanted[k].first); out != nullptr) {
+                for (size_t i = 0; i < s; ++i) {
+                    out[scatter[i]] = tmp[k * s + i];
+                }
             }
-            return NGX_OK;
-        };
-        int rc = put(r->src_sum, o.src_f64 + at);
-        if (rc == NGX_OK) rc = put(r->src_max, o.src_f64 + total + at);
-        if (rc == NGX_OK) rc = put(r->src_sum_inverse, o.src_f64 + 2 * total + at);
-        if (rc == NGX_OK) rc = put(r->src_unreachable, o.src_u64 + at);
-        if (rc == NGX_OK) rc = put(r->src_arcs, o.src_u64 + total + at);
-        return rc;
+        }
+        return NGX_OK;
     }
     if (s > 0) {
         if (r->src_sum != nullptr) NGX_CUDA_TRY(cudaMemcpyAsync(r->src_sum, o.src_f64 + at, s * 8, cudaMemcpyDeviceToHost, g->stream));
@@ -781,7 +795,6 @@ int run_apsp(ngx_graph* g, const ngx_apsp_opts* caller_opts, ngx_apsp_result* re
     }
     cudaStreamSynchronize(g->stream);
     free_outputs(g, o);
-    cudaStreamSynchronize(g->stream);
     return rc;
 }
 
