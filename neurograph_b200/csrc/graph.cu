@@ -189,6 +189,7 @@ void release(ngx_graph* g) {
     cudaFree(g->d_persistent);
     cudaFree(g->d_call_out);
     cudaFree(g->d_call_dag);
+    cudaFree(g->d_landmarks);
     if (g->graph_exec != nullptr) {
         cudaGraphExecDestroy(static_cast<cudaGraphExec_t>(g->graph_exec));
     }

@@ -106,6 +106,9 @@ struct ngx_graph {
     size_t call_out_bytes = 0;
     void* d_call_dag = nullptr;
     size_t call_dag_bytes = 0;
+    // distances from and to the landmarks of a run (2 * kTile * n doubles), computed by each run that uses them
+    void* d_landmarks = nullptr;
+    size_t landmarks_bytes = 0;
 
     // bucket width per size class (floor(log2 n)), as a multiple of each graph's mean arc length (ngx_batch_autotune)
     double class_scale[64] = {};

@@ -42,6 +42,12 @@ struct TileJob {
     int64_t n_max = 0;                 // largest graph (workspace slot size)
     int64_t num_arcs = 0;              // stored arcs of the job's graphs
     double plain_delta = 1.0;          // bucket width of the plain form (single graph)
+    // single-graph runs with landmark bounds; a landmark run writes its distance rows to `rows`, over the reverse arcs
+    // when `reverse`
+    const double* landmark_from = nullptr;
+    const double* landmark_to = nullptr;
+    double* rows = nullptr;
+    bool reverse = false;
     bool track_reach = false;          // keep per-tile reach lists (a graph of several strongly connected components)
 };
 

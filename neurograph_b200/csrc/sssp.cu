@@ -340,8 +340,10 @@ int launch_tiles(ngx_graph* g, const ngx_apsp_opts* opts, int tile_mode, const T
     unsigned long long* group_ws = reinterpret_cast<unsigned long long*>(ws);
     ws += static_cast<size_t>(slots) * group_bytes;
     SsspParams p{};
-    p.g = g->csr(opts->metric);
+    p.g = job.reverse ? g->reverse_csr() : g->csr(opts->metric);
     p.g.n = n;
+    p.landmark_from = job.landmark_from;
+    p.landmark_to = job.landmark_to;
     p.sources = o.sources;
     p.num_sources = job.num_sources;
     p.num_tiles = num_tiles;
@@ -436,7 +438,7 @@ int launch_tiles(ngx_graph* g, const ngx_apsp_opts* opts, int tile_mode, const T
     p.out.src_inv = o.src_f64 + 2 * job.num_sources;
     p.out.src_unreach = o.src_u64;
     p.out.src_arcs = o.src_u64 + job.num_sources;
-    p.out.rows = o.rows;
+    p.out.rows = job.rows != nullptr ? job.rows : o.rows;
 
     if (synchronous) {
         if (g->run_start == nullptr) {
@@ -663,7 +665,7 @@ int read_totals(ngx_graph* g, const RunOutputs& o, std::vector<unsigned long lon
 
 // One single-graph run of `sources` (graph 0 of the handle).
 int run_sources(ngx_graph* g, const ngx_apsp_opts* opts, int tile_mode, const std::vector<int32_t>& sources, int64_t hist_bins, double hist_max,
-                bool want_rows, DagOutputs* extra, RunOutputs& o, float* ms) {
+                bool want_rows, DagOutputs* extra, RunOutputs& o, float* ms, const TileJob* with = nullptr) {
     const int64_t num_sources = static_cast<int64_t>(sources.size());
     if (const int rc = alloc_outputs(g, 1, num_sources, hist_bins, want_rows, o, false); rc != NGX_OK) {
         return rc;
@@ -675,7 +677,7 @@ int run_sources(ngx_graph* g, const ngx_apsp_opts* opts, int tile_mode, const st
     NGX_CUDA_TRY(cudaMemsetAsync(o.block, 0, o.zeroed_bytes, g->stream));
     NGX_CUDA_TRY(cudaMemcpyAsync(o.graphs, &desc, sizeof(desc), cudaMemcpyHostToDevice, g->stream));
     NGX_CUDA_TRY(cudaMemcpyAsync(o.sources, sources.data(), sizeof(int32_t) * sources.size(), cudaMemcpyHostToDevice, g->stream));
-    TileJob job;
+    TileJob job = with != nullptr ? *with : TileJob{};  // (its landmark fields)
     job.num_graphs = 1;
     job.num_items = (num_sources + kTile - 1) / kTile;
     job.d_items = nullptr;
@@ -685,6 +687,56 @@ int run_sources(ngx_graph* g, const ngx_apsp_opts* opts, int tile_mode, const st
     job.plain_delta = delta;
     job.track_reach = g->scc_components > 1;
     return launch_tiles(g, opts, tile_mode, job, hist_bins, hist_max, o, extra, ms, true);
+}
+
+// Whether a run of `tiles` source tiles pays for landmark bounds: two more tiles, each run by itself, and memory for
+// 2 x kTile rows.
+//  * Twelve waves or more: in fewer, the two extra tiles take as long as they save (two waves' time at 2000 vertices).
+//  * Lengths that spread: mean(len) x mean(1 / len) is 1 for equal lengths, 1.3 and 2.7 for log-normal weights of sigma 0.5
+//    and 1, 1.6 for integers up to 10. Measured kernel times without and with: sigma 1, APSP of 148 tiles on 100,000
+//    vertices 181 and 158 ms, Brandes of 74 tiles 108 and 102 ms, APSP of 938 tiles on 30,000 vertices 267 and 240 ms;
+//    sigma 0.5, gradient of 128 tiles 115 and 118 ms; integers 60.5 and 60.2; unit weights 125.4 and 126.4.
+//  * A strongly connected graph (tiles with reach lists start without bounds) of filtered vertices, the regular metric
+//    (the reverse arcs have no other lengths), and an eighth of the workspace memory.
+bool landmarks_pay(const ngx_graph* g, const ngx_apsp_opts* opts, int64_t tiles) {
+    const GraphPart& part = g->parts[0];
+    if (opts->mode != NGX_MODE_BATCHED || opts->metric != NGX_METRIC_REGULAR || opts->max_iterations != 0 || g->scc_components != 1 ||
+        g->m_stored < kFilterDegree * g->n || part.mean_len_regular * part.mean_len_inverse < 2.0) {
+        return false;
+    }
+    const int64_t resident = 2 * static_cast<int64_t>(g->sm_count);  // the default launch shape
+    const int group = choose_group_size(opts->tile_ctas, resident, tiles, resident, static_cast<double>(g->n),
+                                        static_cast<double>(g->m_stored) / static_cast<double>(g->n));
+    return tiles >= 12 * (resident / group) && 2 * static_cast<size_t>(kTile) * static_cast<size_t>(g->n) * sizeof(double) <= workspace_budget(g) / 8;
+}
+
+// Distances from and to kTile landmarks spread over the vertex ids, for the tiles' first bounds (landmark_bounds): one tile
+// over the forward arcs and one over the reverse arcs.
+int compute_landmarks(ngx_graph* g, const ngx_apsp_opts* opts, TileJob* with, float* ms) {
+    const size_t rows = static_cast<size_t>(kTile) * static_cast<size_t>(g->n);
+    if (const int rc = grow_buffer(g, &g->d_landmarks, &g->landmarks_bytes, 2 * rows * sizeof(double)); rc != NGX_OK) {
+        return rc;
+    }
+    std::vector<int32_t> landmarks(kTile);
+    for (int64_t l = 0; l < kTile; ++l) {
+        landmarks[static_cast<size_t>(l)] = static_cast<int32_t>((2 * l + 1) * g->n / (2 * kTile));
+    }
+    ngx_apsp_opts plain = *opts;
+    plain.tile_ctas = 0;
+    for (int to = 0; to < 2; ++to) {
+        TileJob job;
+        job.rows = static_cast<double*>(g->d_landmarks) + (to != 0 ? rows : 0);
+        job.reverse = to != 0;
+        RunOutputs o;
+        const int rc = run_sources(g, &plain, kModeApsp, landmarks, 0, 0.0, false, nullptr, o, ms, &job);
+        free_outputs(g, o);
+        if (rc != NGX_OK) {
+            return rc;
+        }
+    }
+    with->landmark_from = static_cast<const double*>(g->d_landmarks);
+    with->landmark_to = with->landmark_from + rows;
+    return NGX_OK;
 }
 
 // Histogram bound when the caller gives none: 1.5 x the largest eccentricity of up to one tile of sources spread
@@ -777,7 +829,18 @@ int run_apsp(ngx_graph* g, const ngx_apsp_opts* caller_opts, ngx_apsp_result* re
     }
     RunOutputs o;
     float ms = 0.0f;
-    int rc = run_sources(g, opts, tile_mode, sources, hist_bins, hist_max, rows != nullptr, extra, o, &ms);
+    TileJob with;
+    if (landmarks_pay(g, opts, (num_sources + kTile - 1) / kTile)) {
+        const int rc_l = compute_landmarks(g, opts, &with, &ms);
+        if (rc_l == NGX_OUT_OF_MEMORY || rc_l == NGX_TIMEOUT) {
+            cudaGetLastError();  // the run does without
+            set_last_error("");
+            with = TileJob{};
+        } else if (rc_l != NGX_OK) {
+            return rc_l;
+        }
+    }
+    int rc = run_sources(g, opts, tile_mode, sources, hist_bins, hist_max, rows != nullptr, extra, o, &ms, &with);
     if (rc == NGX_OK) {
         std::vector<unsigned long long> acc, counters;
         rc = read_totals(g, o, acc, counters);

@@ -63,6 +63,9 @@ struct SsspParams {
     int64_t num_tiles;             // work items
     double delta;
     const GraphDesc* graphs;       // batch table (tile kernel)
+    // distances from and to the landmarks, kTile rows of num_vertices each (nullptr: none), see landmark_bounds
+    const double* landmark_from;
+    const double* landmark_to;
     const WorkItem* items;         // work items in scheduling order, or nullptr: tile t of graph 0
     unsigned long long max_iterations;  // per tile
     unsigned long long* tile_counter;
@@ -339,11 +342,12 @@ __device__ __forceinline__ void batched_expand(TileSmem& sh, WarpScratch& w, War
     const Arc* const arcs = sh.args.arcs + entry.beg;
     const int64_t vrow = static_cast<int64_t>(entry.v) * kTile + lane;
     const unsigned long long row_bits = __ldcg(&dist[vrow]);
+    const int old_bound = ld_bound(&sh.args.bound[entry.v]);
     const uint32_t row_hi = static_cast<uint32_t>(row_bits >> 32);
     const int bound_base = sh.args.bound_base;
     const uint32_t row_max = __reduce_max_sync(kFullMask, lane < sh.args.nsrc ? row_hi : 0u);
     const int max_key = bound_key(row_max, bound_base);
-    if (lane == 0 && max_key < kNoBound) {
+    if (lane == 0 && max_key < old_bound) {
         sh.args.bound[entry.v] = static_cast<uint8_t>(max_key > 0 ? max_key : 0);
     }
     const uint32_t min_hi = __reduce_min_sync(kFullMask, ((amask >> lane) & 1u) != 0u ? row_hi : 0xFFFFFFFFu);
@@ -833,6 +837,32 @@ __device__ __forceinline__ void compact_queue(const uint32_t* pend, int32_t* q, 
     }
 }
 
+// The tile's first bounds, from kTile landmarks: d[x][s] <= d(s, l) + d(l, x) for every landmark l, so the smallest over l of
+// max_s d(s, l) + d(l, x) bounds the row of x before any of its sources has reached it. Rounded sums over at most 2^31
+// arcs differ from the exact path length by less than 2^-21 of it each way; the factor covers all of them. reach is
+// shared memory. The caller separates this from the expansions by a group barrier.
+__device__ __forceinline__ void landmark_bounds(const SsspParams& p, int64_t n, const int* s_src, int nsrc, unsigned long long* reach, uint8_t* bound,
+                                                int bound_base, int64_t first, int64_t stride) {
+    if (threadIdx.x < kTile) {
+        reach[threadIdx.x] = 0ull;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < kTile * nsrc; i += blockDim.x) {
+        const int l = i & (kTile - 1);
+        atomicMax(&reach[l], static_cast<unsigned long long>(__double_as_longlong(__ldg(&p.landmark_to[l * n + s_src[i / kTile]]))));
+    }
+    __syncthreads();
+    for (int64_t x = first; x < n; x += stride) {
+        double least = INFINITY;
+#pragma unroll 8
+        for (int l = 0; l < kTile; ++l) {
+            least = fmin(least, __longlong_as_double(static_cast<long long>(reach[l])) + __ldg(&p.landmark_from[l * n + x]));
+        }
+        const int key = bound_key(static_cast<uint32_t>(__double2hiint(least * (1.0 + 0x1p-20))), bound_base);
+        bound[x] = static_cast<uint8_t>(key < 0 ? 0 : (key < kNoBound ? key : kNoBound));
+    }
+}
+
 // kMulti: the launch may put several CTAs on a tile (p.group_size > 1, cooperative launch); without it the group is
 // the CTA itself, whose control block lives in shared memory. kReach: the tiles keep reach lists.
 template <int kMode, int kUnroll, int kBlock, int kMinBlocks, bool kMulti = false, bool kReach = false>
@@ -1002,6 +1032,13 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
                                   NGX_GWARPS, static_cast<int>(n), gd.m < kFilterDegree * gd.n ? 1 : 0 };
         }
         __syncthreads();
+        if (!kReach && p.landmark_from != nullptr) {
+            landmark_bounds(p, n, s_src, nsrc, s_max, bound, sh.args.bound_base, NGX_GT, NGX_GTHREADS);
+            __syncthreads();
+            if (tid < kTile) {
+                s_max[tid] = 0ull;
+            }
+        }
         if ((!kMulti || grp().rank == 0) && warp == 0) {
             const int v = s_src[lane];
             if (v >= 0) {
