@@ -71,7 +71,7 @@ std::vector<GraphDesc> graph_table(const ngx_graph* g, int metric, double delta_
     for (size_t i = 0; i < g->parts.size(); ++i) {
         const GraphPart& part = g->parts[i];
         const double scale = delta_scale > 0.0 ? delta_scale : (g->class_scale[size_class(part.n)] > 0.0 ? g->class_scale[size_class(part.n)]
-                                                                                     : default_delta_scale(part.n, part.m_stored));
+                                                                                     : default_delta_scale(part));
         const double mean = metric == NGX_METRIC_INVERSE ? part.mean_len_inverse : part.mean_len_regular;
         descs[i] = GraphDesc{ part.n, part.m_stored, part.row_off, part.vertex_off, part.n, part.vertex_off, pick_delta(mean, 0.0, scale) };
     }
@@ -459,7 +459,7 @@ int ngx_batch_autotune(ngx_graph* g, int task, double* class_scales) {
             }
             double best_rate = -1.0, best_scale = 1.0;
             const GraphPart& probe_part = g->parts[static_cast<size_t>(probe[static_cast<size_t>(c)])];
-            const double own = default_delta_scale(probe_part.n, probe_part.m_stored);  // the untuned width, tried too
+            const double own = default_delta_scale(probe_part);  // the untuned width, tried too
             for (const double scale : { own, kScales[0], kScales[1], kScales[2], kScales[3], kScales[4], kScales[5] }) {
                 double rate = 0.0;
                 if (const int rc = time_wave(g, mode, probe[static_cast<size_t>(c)], scale, aopts, &rate); rc != NGX_OK) {
@@ -503,8 +503,8 @@ int ngx_batch_autotune(ngx_graph* g, int task, double* class_scales) {
             }
             int best_group = 1;
             for (const int gs : { 0, 2, 4 }) {
-                // groups of several CTAs per tile run with the default block shape; 0 = the library's own rule (by L2
-                // residency and the slots memory affords), which is what a run with tile_ctas 0 gets
+                // groups of several CTAs per tile run with the default block shape; 0 = the library's own rule (by graph
+                // size, density and waves, and the slots memory affords), which is what a run with tile_ctas 0 gets
                 aopts.block_threads = kShapes[0].block;
                 aopts.ctas_per_sm = kShapes[0].per_sm;
                 aopts.tile_ctas = gs;

@@ -79,7 +79,7 @@ int ngx_graph_autotune(ngx_graph* g, int task, int64_t sample_sources, ngx_tunin
         const int64_t wave = static_cast<int64_t>(g->sm_count) * 2 * kTile;
         const int64_t k = std::min<int64_t>(g->n, sample_sources > 0 ? sample_sources : wave);
         if (k == 0) {
-            t.delta_scale = default_delta_scale(g->parts[0].n, g->parts[0].m_stored);
+            t.delta_scale = degree_delta_scale(g->parts[0].n, g->parts[0].m_stored);
             t.block_threads = 512;
             t.ctas_per_sm = 2;
             t.tile_ctas = 1;
@@ -90,8 +90,9 @@ int ngx_graph_autotune(ngx_graph* g, int task, int64_t sample_sources, ngx_tunin
         }
         const std::vector<int64_t> sources(g->source_order.begin(), g->source_order.begin() + k);
         const double mean = g->parts[0].mean_len_regular;
-        // bucket widths: the library's default for this graph's degree first, then fixed multiples of the mean length
-        const double kScales[] = { default_delta_scale(g->parts[0].n, g->parts[0].m_stored), 0.125, 0.25, 0.5, 1.0, 2.0 };
+        // bucket widths: the width by the graph's degree first, then fixed multiples of the mean length (2 x, which sparse
+        // graphs and little spread want, among them)
+        const double kScales[] = { degree_delta_scale(g->parts[0].n, g->parts[0].m_stored), 0.125, 0.25, 0.5, 1.0, 2.0 };
         static const Shape kShapes[] = { { 512, 2 }, { 384, 2 }, { 256, 3 }, { 256, 4 } };
         const int tiles = static_cast<int>((k + kTile - 1) / kTile);
         // CTAs per tile: the library's own choice (0: the bucket-width trials run with it, as untuned runs do), 1, 2,
