@@ -1215,6 +1215,10 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
                 }
                 for (int64_t i = NGX_GT; i < nt; i += NGX_GTHREADS) {
                     lvl[i] = kNoLevel;
+                    delta[i] = 0.0;  // pairs that no level releases keep it (see below)
+                    if constexpr (kMode == kModeGrad) {
+                        delta_g[i] = 0.0;
+                    }
                 }
             }
             sync([&](volatile TileShared& c) {
@@ -1276,6 +1280,20 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
                     c.level = level + 1u;
                     loff[level + 1u] = start + len;
                 });
+            }
+            // Arcs that vanish against their distances (fl(d + len) == d) close cycles, whose pairs, and those behind them,
+            // no level releases: they have no path count and their dependency is 0. No level writes it, so it is stored here;
+            // a tile without such pairs (all listed) pays for one comparison.
+            if (!tree && static_cast<unsigned long long>(s.lvl_start) < s.active_pairs + static_cast<unsigned long long>(nsrc)) {
+                for (int64_t i = NGX_GT; i < nt; i += NGX_GTHREADS) {
+                    if (__ldcg(&cnt[i]) != 0u) {
+                        delta[i] = 0.0;
+                        if constexpr (kMode == kModeGrad) {
+                            delta_g[i] = 0.0;
+                        }
+                    }
+                }
+                sync0();
             }
             if (tid == 0) {
                 const long long now = clock64();
