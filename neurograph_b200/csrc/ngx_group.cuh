@@ -67,8 +67,9 @@ struct Group {
     // Barrier of the group. The last CTA to arrive runs update(*ctl) on its thread 0; then every CTA copies the
     // control block into `local` (its shared memory). bar_target is the CTA's count of barriers passed (shared). A
     // CTA that gave up waiting is out of the group for the rest of the launch: its bar_target becomes kGroupLeft, it
-    // joins no later barrier, and its local control block is halted (Ctl::halt: no work left), so it runs to the end
-    // of the kernel without touching the group's state; the run then reports NGX_TIMEOUT.
+    // joins no later barrier, and its local control block is halted (Ctl::halt: no work left). What the CTAs do between
+    // this barrier and the next may stay undone from then on, so it must leave its loops here and end, without a look at the
+    // group's state; the others give up at the next barrier. The run then reports NGX_TIMEOUT.
     template <typename Update>
     __device__ __forceinline__ void sync(Ctl& local, unsigned& bar_target, Update&& update) const {
         __syncthreads();
@@ -154,6 +155,9 @@ __device__ __forceinline__ unsigned long long group_exclusive_scan(const Group<C
     unsigned long long base = 0, total = 0;
     if (grp.size > 1) {
         grp.sync(local, bar_target);
+        if (bar_target == kGroupLeft) {
+            return ~0ull;  // left the group: the others' partial sums may be missing
+        }
         // every CTA adds the chunks before its own (at most a few hundred words, read by one thread)
         if (tid == 0) {
             unsigned long long before = 0, all = 0;

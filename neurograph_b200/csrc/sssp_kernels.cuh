@@ -905,6 +905,10 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
         }
     };
     const auto sync0 = [&]() { sync([](volatile TileShared&) {}); };
+    // A CTA that gave up at a barrier (Group::sync) has no work and no complete state of the others': parents, counts and lists
+    // may be words nobody wrote. The distance phase finds it halted; the DAG phase and the epilogue leave the tile loop, and
+    // with it the kernel, after the barrier at which it gave up. Always false for single-CTA tiles.
+    const auto left = [&]() { return kMulti && s.stop != 0; };
     // this thread's (warp's) index among the group's threads (warps), and their counts
 #define NGX_GT (kMulti ? static_cast<int64_t>(blockIdx.x % p.group_size) * blockDim.x + threadIdx.x : static_cast<int64_t>(threadIdx.x))
 #define NGX_GTHREADS (kMulti ? static_cast<int64_t>(p.group_size) * blockDim.x : static_cast<int64_t>(blockDim.x))
@@ -1171,8 +1175,14 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
             uint32_t* const low = stamp;  // its words held the distance phase's bounds until here
             dag_low(dist, low, n, nsrc, lane, NGX_GW, NGX_GWARPS);
             sync0();
+            if (left()) {
+                break;
+            }
             dag_count<kMode == kModeGrad>(low, lane < nsrc ? s_src[lane] : -1, sigma, cnt, scnt, pred, lvl, ctl(), NGX_GW);
             sync0();
+            if (left()) {
+                break;
+            }
             // when every reached pair has exactly one DAG predecessor (as many DAG arcs as reached non-source pairs) the
             // DAGs are trees
             tree = s.dag_arcs == s.active_pairs && b.succ_capacity > 0;
@@ -1185,6 +1195,9 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
             }
             dag_tree_walk(cnt, lvl, scnt, reinterpret_cast<unsigned long long*>(sigma), s_src, NGX_GW);
             sync0();
+            if (left()) {
+                break;
+            }
             if (tid == 0) {
                 if (!kMulti || grp().rank == 0) {
                     atomicAdd(&cnts[kDagEntries], s.active_pairs + static_cast<unsigned long long>(nsrc));
@@ -1195,11 +1208,17 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
             }
           } else {
             const unsigned long long dag_arcs = group_exclusive_scan(grp(), s, s_bar, scnt, soff, nt, s_part);
+            if (left()) {
+                break;
+            }
             const bool use_lists = dag_arcs <= static_cast<unsigned long long>(b.succ_capacity);
             for (int64_t i = NGX_GT; i < nt; i += NGX_GTHREADS) {
                 scnt[i] = 0u;
             }
             sync0();
+            if (left()) {
+                break;
+            }
             if (use_lists) {
                 if (kMode == kModeBrandes || tree) {
                     dag_fill<true>(b.arc_src, low, cnt, pred, soff, scnt, succ, NGX_GW);
@@ -1207,6 +1226,9 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
                     dag_fill<false>(b.arc_src, low, cnt, pred, soff, scnt, succ, NGX_GW);
                 }
                 sync0();
+                if (left()) {
+                    break;
+                }
                 dag_sort(soff, succ, nt, NGX_GT, NGX_GTHREADS);
             }
             if (!use_lists) {
@@ -1231,6 +1253,9 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
                 c.next_len = 0;
                 loff[0] = 0;
             });
+            if (left()) {
+                break;
+            }
             if (tid == 0) {
                 const long long now = clock64();
                 atomicAdd(&cnts[kCyclesCount], static_cast<unsigned long long>(now - t_phase));
@@ -1256,6 +1281,9 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
                 }
             }
             sync0();
+            if (left()) {
+                break;
+            }
           if (use_lists) {
             // --- sigma and delta over the successor lists. In a tree every sigma is 1 and every child is released by its
             // only parent, so the sigma levels need neither sums nor counts.
@@ -1280,6 +1308,12 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
                     c.level = level + 1u;
                     loff[level + 1u] = start + len;
                 });
+                if (left()) {
+                    break;
+                }
+            }
+            if (left()) {
+                break;
             }
             // Arcs that vanish against their distances (fl(d + len) == d) close cycles, whose pairs, and those behind them,
             // no level releases: they have no path count and their dependency is 0. No level writes it, so it is stored here;
@@ -1294,6 +1328,9 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
                     }
                 }
                 sync0();
+                if (left()) {
+                    break;
+                }
             }
             if (tid == 0) {
                 const long long now = clock64();
@@ -1313,6 +1350,12 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
                                                   reinterpret_cast<double*>(s_acc_sum), lane, warp, NGX_GW, NGX_GWARPS);
                 }
                 sync0();
+                if (left()) {
+                    break;
+                }
+            }
+            if (left()) {
+                break;
             }
             if (tid == 0) {
                 if ((!kMulti || grp().rank == 0)) {
@@ -1352,6 +1395,12 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
                     c.level = level + 1u;
                     loff[level + 1u] = start + len;
                 });
+                if (left()) {
+                    break;
+                }
+            }
+            if (left()) {
+                break;
             }
             if (tid == 0) {
                 const long long now = clock64();
@@ -1369,6 +1418,12 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
                                                    b.grad_cpl, b.grad_eff);
                 }
                 sync0();
+                if (left()) {
+                    break;
+                }
+            }
+            if (left()) {
+                break;
             }
             if (tid == 0) {
                 if ((!kMulti || grp().rank == 0)) {
@@ -1500,6 +1555,9 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
                 atomicMax(&g_acc[2 * kTile * kAccDigits + 2 * kTile + tid], s_max[tid]);
             }
             sync0();
+            if (left()) {
+                break;
+            }
             if ((!kMulti || grp().rank == 0)) {
                 for (int i = tid; i < 2 * kTile * kAccDigits; i += blockDim.x) {
                     smem[i] = __ldcg(&g_acc[i]);
