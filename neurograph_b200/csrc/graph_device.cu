@@ -17,6 +17,7 @@
 #include <cstring>
 #include <string>
 #include <thread>
+#include <utility>
 
 #include "ngx_common.cuh"
 #include "ngx_graph.h"
@@ -388,9 +389,16 @@ int update_weights_on_device(ngx_graph* g, const double* w) {
     }
     cudaStream_t s = g->stream;
     if (g->d_stored_of_user == nullptr) {
-        // a host-built handle keeps the map on the host: upload it once
-        NGX_CUDA_TRY(cudaMalloc(&g->d_stored_of_user, static_cast<size_t>(m_user) * 4));
-        NGX_CUDA_TRY(cudaMemcpyAsync(g->d_stored_of_user, g->stored_of_user.data(), static_cast<size_t>(m_user) * 4, cudaMemcpyHostToDevice, s));
+        // a host-built handle keeps the map on the host: upload it once. The handle gets it when it is there: a map that was
+        // not copied would be taken for stored indices by the next update.
+        struct DeviceMap {
+            int32_t* p = nullptr;
+            ~DeviceMap() { cudaFree(p); }
+        } map;
+        NGX_CUDA_TRY(cudaMalloc(&map.p, static_cast<size_t>(m_user) * 4));
+        NGX_CUDA_TRY(cudaMemcpyAsync(map.p, g->stored_of_user.data(), static_cast<size_t>(m_user) * 4, cudaMemcpyHostToDevice, s));
+        NGX_CUDA_TRY(cudaStreamSynchronize(s));
+        std::swap(g->d_stored_of_user, map.p);
     }
     // the weights and the check's results in the handle's call buffer (a run that follows reuses it in stream order)
     if (const int rc = grow_buffer(g, &g->d_call_out, &g->call_out_bytes, 32 + static_cast<size_t>(m_user) * 8); rc != NGX_OK) {
