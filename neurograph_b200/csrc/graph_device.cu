@@ -209,7 +209,7 @@ struct Carver {
     }
 };
 
-// The build's temporary block, freed on every exit.
+// A temporary block of the build, freed on every exit.
 struct TempBlock {
     void* p = nullptr;
     ~TempBlock() { cudaFree(p); }
@@ -250,32 +250,26 @@ int build_graph_on_device(const ngx_csr* csr, ngx_graph* g) {
         }
     } joiner{ sums_thread };
 
-    // every array's size is known up front (no more arcs are stored than given)
+    // three blocks: what is needed to count the stored arcs, and, once they are counted (zero weights are not stored), the
+    // handle's arrays and the sort's
     const size_t mu = static_cast<size_t>(m_user);
     int64_t* d_user_rows = nullptr;
     int32_t* d_col = nullptr;
     double* d_w = nullptr;
-    int64_t* d_kept = nullptr;
+    int64_t *d_kept = nullptr, *d_rows = nullptr;
     unsigned long long* d_red = nullptr;  // bad arc, max degree, min length bits, max length bits
-    uint32_t *d_target = nullptr, *d_target_sorted = nullptr;  // unsigned keys: the sort looks at the low bits only
-    int32_t *d_index = nullptr, *d_index_sorted = nullptr;
-    char *d_scan = nullptr, *d_sort = nullptr;
-    size_t scan_bytes = 0, sort_bytes = 0;
-    NGX_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, d_kept, g->d_row_ptr, n + 1, s));
-    NGX_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, d_target, d_target_sorted, d_index, d_index_sorted, m_user, 0, bits_for(n), s));
+    char* d_scan = nullptr;
+    size_t scan_bytes = 0;
+    NGX_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, d_kept, d_rows, n + 1, s));
     TempBlock tmp;
     Carver temps;
     temps.take(&d_user_rows, static_cast<size_t>(n) + 1);
     temps.take(&d_col, mu);
     temps.take(&d_w, mu);
     temps.take(&d_kept, static_cast<size_t>(n) + 1);
+    temps.take(&d_rows, static_cast<size_t>(n) + 1);
     temps.take(&d_red, 4);
-    temps.take(&d_target, mu);
-    temps.take(&d_index, mu);
-    temps.take(&d_target_sorted, mu);
-    temps.take(&d_index_sorted, mu);
     temps.take(&d_scan, scan_bytes);
-    temps.take(&d_sort, sort_bytes);
     if (const int rc = temps.allocate(&tmp.p); rc != NGX_OK) {
         return rc;
     }
@@ -290,8 +284,12 @@ int build_graph_on_device(const ngx_csr* csr, ngx_graph* g) {
     const int row_grid = grid_for(n * 32, kBuildBlock, g->sm_count);
     count_rows_kernel<<<row_grid, kBuildBlock, 0, s>>>(d_user_rows, d_col, d_w, n, d_kept, d_red, d_red + 1, d_red + 2, d_red + 3);
     NGX_CUDA_TRY(cudaGetLastError());
+    // stored row offsets: exclusive sum of the kept counts (n + 1 entries, the last one m)
+    NGX_CUDA_TRY(cub::DeviceScan::ExclusiveSum(d_scan, scan_bytes, d_kept, d_rows, n + 1, s));
     unsigned long long red[4];
+    int64_t m = 0;
     NGX_CUDA_TRY(cudaMemcpyAsync(red, d_red, sizeof(red), cudaMemcpyDeviceToHost, s));
+    NGX_CUDA_TRY(cudaMemcpyAsync(&m, d_rows + n, 8, cudaMemcpyDeviceToHost, s));
     NGX_CUDA_TRY(cudaStreamSynchronize(s));
     if (red[0] != ~0ull) {
         const int64_t e = static_cast<int64_t>(red[0]);
@@ -300,23 +298,34 @@ int build_graph_on_device(const ngx_csr* csr, ngx_graph* g) {
                                               (bad_target ? " has an out-of-range target" : " has a non-finite weight"));
     }
 
+    const size_t ms = static_cast<size_t>(m);
     Carver arrays;
     arrays.take(&g->d_row_ptr, static_cast<size_t>(n) + 1);
     arrays.take(&g->d_rrow_ptr, static_cast<size_t>(n) + 1);
-    arrays.take(&g->d_arcs_regular, mu);
-    arrays.take(&g->d_arcs_inverse, mu);
-    arrays.take(&g->d_rarcs, mu);
-    arrays.take(&g->d_arc_src, mu);
+    arrays.take(&g->d_arcs_regular, ms);
+    arrays.take(&g->d_arcs_inverse, ms);
+    arrays.take(&g->d_rarcs, ms);
+    arrays.take(&g->d_arc_src, ms);
     arrays.take(&g->d_stored_of_user, mu);
     if (const int rc = arrays.allocate(&g->d_block); rc != NGX_OK) {
         return rc;
     }
-    // stored row offsets: exclusive sum of the kept counts (n + 1 entries, the last one m)
-    NGX_CUDA_TRY(cub::DeviceScan::ExclusiveSum(d_scan, scan_bytes, d_kept, g->d_row_ptr, n + 1, s));
-    int64_t m = 0;
-    NGX_CUDA_TRY(cudaMemcpyAsync(&m, g->d_row_ptr + n, 8, cudaMemcpyDeviceToHost, s));
-    NGX_CUDA_TRY(cudaStreamSynchronize(s));
-
+    uint32_t *d_target = nullptr, *d_target_sorted = nullptr;  // unsigned keys: the sort looks at the low bits only
+    int32_t *d_index = nullptr, *d_index_sorted = nullptr;
+    char* d_sort = nullptr;
+    size_t sort_bytes = 0;
+    NGX_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, d_target, d_target_sorted, d_index, d_index_sorted, m, 0, bits_for(n), s));
+    TempBlock sort_tmp;
+    Carver sort_temps;
+    sort_temps.take(&d_target, ms);
+    sort_temps.take(&d_index, ms);
+    sort_temps.take(&d_target_sorted, ms);
+    sort_temps.take(&d_index_sorted, ms);
+    sort_temps.take(&d_sort, sort_bytes);
+    if (const int rc = sort_temps.allocate(&sort_tmp.p); rc != NGX_OK) {
+        return rc;
+    }
+    NGX_CUDA_TRY(cudaMemcpyAsync(g->d_row_ptr, d_rows, (static_cast<size_t>(n) + 1) * 8, cudaMemcpyDeviceToDevice, s));
     fill_rows_kernel<<<row_grid, kBuildBlock, 0, s>>>(d_user_rows, d_col, d_w, n, g->d_row_ptr, g->d_arcs_regular, g->d_arcs_inverse, g->d_arc_src,
                                                       g->d_stored_of_user, d_target, d_index);
     NGX_CUDA_TRY(cudaGetLastError());
@@ -330,17 +339,6 @@ int build_graph_on_device(const ngx_csr* csr, ngx_graph* g) {
     }
     NGX_CUDA_TRY(cub::DeviceScan::ExclusiveSum(d_scan, scan_bytes, d_kept, g->d_rrow_ptr, n + 1, s));
     if (m > 0) {
-        // the temporary storage was sized for m_user pairs; fewer (zero weights dropped) should need no more
-        TempBlock more;
-        if (m != m_user) {
-            size_t need = 0;
-            NGX_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, need, d_target, d_target_sorted, d_index, d_index_sorted, m, 0, bits_for(n), s));
-            if (need > sort_bytes) {
-                NGX_CUDA_TRY(cudaMalloc(&more.p, need));
-                d_sort = static_cast<char*>(more.p);
-                sort_bytes = need;
-            }
-        }
         NGX_CUDA_TRY(cub::DeviceRadixSort::SortPairs(d_sort, sort_bytes, d_target, d_target_sorted, d_index, d_index_sorted, m, 0, bits_for(n), s));
         reverse_records_kernel<<<grid_for(m, kBuildBlock, g->sm_count), kBuildBlock, 0, s>>>(d_index_sorted, m, g->d_arcs_regular, g->d_arc_src,
                                                                                             g->d_rarcs);
