@@ -13,7 +13,7 @@
 //            component); the vertices of its colour that reach it are its component, found backwards: a vertex joins
 //            when one of its out-neighbours of the same colour has joined.
 // Trim, colour and peel repeat until every vertex has a component. Every pass is a kernel launch; the host
-// reads a change flag after one or a few, so nothing waits on the device beyond one launch.
+// reads the change flags after one or a few, so nothing waits on the device beyond one launch.
 
 #include <cuda_runtime.h>
 
@@ -213,27 +213,33 @@ __global__ void scc_pairs_kernel(int64_t n, const unsigned long long* hist, unsi
     }
 }
 
-// Runs `launch` (which may set *flag) until a pass leaves the flag clear. Every pass that sets it makes progress on a
+// Runs `launch(flag)` (which may set *flag) until a pass leaves its flag clear. Every pass that sets it makes progress on a
 // finite quantity (an assignment, a larger colour, a new member), so n + 1 passes always suffice. Passes after the last
-// change do nothing, so several are launched for each look at the flag (only the last of them matters) where a pass
-// costs less than the round trip to the host: up to 4e6 arcs, about 15 us either way.
+// change do nothing, so several are launched for each look at their flags where a pass costs less than the round trip
+// to the host: up to 4e6 arcs, about 15 us either way. The pre-pass's cap counts the passes up to the first clear flag,
+// as many as one look per pass would take.
+constexpr int kPassesPerLook = 4;
 template <typename Launch>
-int until_stable(ngx_graph* g, int* d_flag, int* h_flag, int64_t max_passes, Launch launch) {
-    const int per_look = g->m_stored <= 4000000 ? 4 : 1;
+int until_stable(ngx_graph* g, int* d_flags, int64_t max_passes, Launch launch) {
+    const int per_look = g->m_stored <= 4000000 ? kPassesPerLook : 1;
+    int flags[kPassesPerLook] = {};
     for (int64_t pass = 0; pass <= max_passes; pass += per_look) {
-        if (g->scc_pass_cap > 0 && (g->scc_passes += per_look) > g->scc_pass_cap) {
-            return fail(NGX_TIMEOUT, "ngx_scc: more passes than the pre-pass allows");
-        }
+        NGX_CUDA_TRY(cudaMemsetAsync(d_flags, 0, per_look * sizeof(int), g->stream));
         for (int i = 0; i < per_look; ++i) {
-            if (i == per_look - 1) {
-                NGX_CUDA_TRY(cudaMemsetAsync(d_flag, 0, sizeof(int), g->stream));
-            }
-            launch();
+            launch(d_flags + i);
         }
         NGX_CUDA_TRY(cudaGetLastError());
-        NGX_CUDA_TRY(cudaMemcpyAsync(h_flag, d_flag, sizeof(int), cudaMemcpyDeviceToHost, g->stream));
+        NGX_CUDA_TRY(cudaMemcpyAsync(flags, d_flags, per_look * sizeof(int), cudaMemcpyDeviceToHost, g->stream));
         NGX_CUDA_TRY(cudaStreamSynchronize(g->stream));
-        if (*h_flag == 0) {
+        int changing = 0;
+        while (changing < per_look && flags[changing] != 0) {
+            ++changing;
+        }
+        const bool stable = changing < per_look;
+        if (g->scc_pass_cap > 0 && (g->scc_passes += changing + (stable ? 1 : 0)) > g->scc_pass_cap) {
+            return fail(NGX_TIMEOUT, "ngx_scc: more passes than the pre-pass allows");
+        }
+        if (stable) {
             return NGX_OK;
         }
     }
@@ -268,7 +274,7 @@ int ngx_scc(ngx_graph* g, int32_t* component, uint64_t* number_components, uint6
         }
         NGX_CUDA_TRY(cudaSetDevice(g->device));
         const size_t words = static_cast<size_t>(n);
-        // device layout: comp i32[n] | color i32[n] | sizes u64[n] | visited u8[n] | flags i32[2], totals u64[3] |
+        // device layout: comp i32[n] | color i32[n] | sizes u64[n] | visited u8[n] | flags i32[kPassesPerLook + 1], totals u64[3] |
         // (size, components) pairs | size histogram u64[n + 1], each 256-byte aligned
         const size_t off_color = align256(words * 4);
         const size_t off_sizes = off_color + align256(words * 4);
@@ -289,7 +295,6 @@ int ngx_scc(ngx_graph* g, int32_t* component, uint64_t* number_components, uint6
         auto* visited = reinterpret_cast<uint8_t*>(base + off_visited);
         auto* flags = reinterpret_cast<int*>(base + off_flags);
         NGX_CUDA_TRY(cudaMemsetAsync(comp, 0xFF, words * 4, g->stream));  // -1: no component yet
-        int h_flag = 0;
         const int vgrid = static_cast<int>(std::min<int64_t>((n + kSccBlock - 1) / kSccBlock, 8 * int64_t(g->sm_count)));
         const bool few_arcs = g->m_stored < 8 * n;
         const int64_t lanes = few_arcs ? kSparseLanes : 32;
@@ -301,36 +306,37 @@ int ngx_scc(ngx_graph* g, int32_t* component, uint64_t* number_components, uint6
         // every round assigns at least the largest unassigned vertex (its own colour's root)
         bool done = false;
         for (int64_t round = 0; round <= n && !done; ++round) {
-            int rc = until_stable(g, flags, &h_flag, n, [&] {
+            int rc = until_stable(g, flags, n, [&](int* flag) {
                 const auto kernel = few_arcs ? scc_trim_kernel<kSparseLanes> : scc_trim_kernel<32>;
-                kernel<<<wgrid, kSccBlock, 0, g->stream>>>(n, row_ptr, arcs, rrow_ptr, rarcs, comp, flags);
+                kernel<<<wgrid, kSccBlock, 0, g->stream>>>(n, row_ptr, arcs, rrow_ptr, rarcs, comp, flag);
             });
             if (rc != NGX_OK) {
                 return rc;
             }
             scc_color_init_kernel<<<vgrid, kSccBlock, 0, g->stream>>>(n, comp, color, visited);
             NGX_CUDA_TRY(cudaGetLastError());
-            rc = until_stable(g, flags, &h_flag, n, [&] {
+            rc = until_stable(g, flags, n, [&](int* flag) {
                 const auto kernel = few_arcs ? scc_color_kernel<kSparseLanes> : scc_color_kernel<32>;
-                kernel<<<wgrid, kSccBlock, 0, g->stream>>>(n, rrow_ptr, rarcs, comp, color, flags);
+                kernel<<<wgrid, kSccBlock, 0, g->stream>>>(n, rrow_ptr, rarcs, comp, color, flag);
             });
             if (rc != NGX_OK) {
                 return rc;
             }
             scc_roots_kernel<<<vgrid, kSccBlock, 0, g->stream>>>(n, comp, color, visited);
             NGX_CUDA_TRY(cudaGetLastError());
-            rc = until_stable(g, flags, &h_flag, n, [&] {
+            rc = until_stable(g, flags, n, [&](int* flag) {
                 const auto kernel = few_arcs ? scc_backward_kernel<kSparseLanes> : scc_backward_kernel<32>;
-                kernel<<<wgrid, kSccBlock, 0, g->stream>>>(n, row_ptr, arcs, comp, color, visited, flags);
+                kernel<<<wgrid, kSccBlock, 0, g->stream>>>(n, row_ptr, arcs, comp, color, visited, flag);
             });
             if (rc != NGX_OK) {
                 return rc;
             }
-            NGX_CUDA_TRY(cudaMemsetAsync(flags + 1, 0, sizeof(int), g->stream));
-            scc_assign_kernel<<<vgrid, kSccBlock, 0, g->stream>>>(n, comp, color, visited, flags + 1);
+            int* const left = flags + kPassesPerLook;  // vertices without a component remain
+            NGX_CUDA_TRY(cudaMemsetAsync(left, 0, sizeof(int), g->stream));
+            scc_assign_kernel<<<vgrid, kSccBlock, 0, g->stream>>>(n, comp, color, visited, left);
             NGX_CUDA_TRY(cudaGetLastError());
             int remaining = 0;
-            NGX_CUDA_TRY(cudaMemcpyAsync(&remaining, flags + 1, sizeof(int), cudaMemcpyDeviceToHost, g->stream));
+            NGX_CUDA_TRY(cudaMemcpyAsync(&remaining, left, sizeof(int), cudaMemcpyDeviceToHost, g->stream));
             NGX_CUDA_TRY(cudaStreamSynchronize(g->stream));
             done = remaining == 0;
         }

@@ -98,3 +98,22 @@ def test_long_chain_runs_without_the_prepass(restatement):
     want = restatement.apsp(csr, sources=sources)
     for k in ("sum", "max", "unreachable", "arcs"):
         assert np.array_equal(got.per_source[k], want["per_source"][k]), k
+
+
+def test_many_stages_within_the_cap():
+    """300 components {i, 599 - i}, every one with arcs to all later ones: the largest id reaches everything, so each stage
+    settles one component and takes five passes (one to trim, two each to colour and to peel). 1500 passes are within the
+    pre-pass's 2048, so the sources are grouped by component, though every vertex has nearer neighbours than its partner."""
+    k = 300
+    n = 2 * k
+    rows, cols, ws = [0], [], []
+    for v in range(n):
+        later = np.arange(min(v, n - 1 - v) + 1, k)
+        t = np.concatenate([[n - 1 - v], later, n - 1 - later])
+        cols.append(t)
+        ws.append(np.concatenate([[50.0], 1.0 + (t[1:] * 7 + v) % 11]))
+        rows.append(rows[-1] + t.size)
+    with ngx.Graph(n, np.array(rows, np.int64), np.concatenate(cols).astype(np.int32), np.concatenate(ws)) as g:
+        order = g.source_order()
+        comp_of = g.scc()["component"][order]
+    assert np.count_nonzero(comp_of[1:] != comp_of[:-1]) == k - 1
