@@ -190,7 +190,8 @@ NGX_API int ngx_graph_request_abort(ngx_graph* graph);
  * with its own events.
  */
 NGX_API int ngx_graph_set_stream(ngx_graph* graph, void* stream);
-/* Caps the device memory the graph's runs may use for workspaces (bytes; 0 = no cap beyond free memory). */
+/* Caps the device memory the graph's runs may use for workspaces, a long run's landmark rows among them (bytes; 0 = no cap
+ * beyond free memory). */
 NGX_API int ngx_graph_set_memory_budget(ngx_graph* graph, uint64_t bytes);
 
 /*

@@ -49,31 +49,52 @@ size_t workspace_budget(const ngx_graph* g) {
     }
     size_t usable = free_bytes + g->workspace_bytes;
     usable = usable > (size_t(1) << 30) ? usable - (size_t(1) << 30) : usable / 2;  // keep 1 GiB headroom
-    if (g->memory_budget != 0 && g->memory_budget < usable) {
-        usable = static_cast<size_t>(g->memory_budget);
+    return std::min(usable, workspace_cap(g));
+}
+
+size_t workspace_cap(const ngx_graph* g) {
+    if (g->memory_budget == 0) {
+        return SIZE_MAX;
     }
-    return usable;
+    const uint64_t rows = g->landmarks_bytes;  // a run's landmark rows are part of its budget
+    return static_cast<size_t>(g->memory_budget > rows ? g->memory_budget - rows : 0);
 }
 
 int ensure_workspace(ngx_graph* g, size_t bytes) {
     if (bytes <= g->workspace_bytes) {
         return NGX_OK;
     }
-    if (g->d_workspace != nullptr) {
-        NGX_CUDA_TRY(cudaStreamSynchronize(g->stream));
-        if (g->graph_exec != nullptr) {
-            // a captured batch run refers to the old workspace
-            cudaGraphExecDestroy(static_cast<cudaGraphExec_t>(g->graph_exec));
-            g->graph_exec = nullptr;
-            g->graph_key = 0;
-        }
-        NGX_CUDA_TRY(cudaFree(g->d_workspace));
-        g->d_workspace = nullptr;
-        g->workspace_bytes = 0;
+    if (const int rc = release_workspace(g); rc != NGX_OK) {
+        return rc;
     }
     NGX_CUDA_TRY(cudaMalloc(&g->d_workspace, bytes));
     g->workspace_bytes = bytes;
     return NGX_OK;
+}
+
+int release_workspace(ngx_graph* g) {
+    if (g->d_workspace == nullptr) {
+        return NGX_OK;
+    }
+    NGX_CUDA_TRY(cudaStreamSynchronize(g->stream));
+    if (g->graph_exec != nullptr) {
+        // a captured batch run refers to the old workspace
+        cudaGraphExecDestroy(static_cast<cudaGraphExec_t>(g->graph_exec));
+        g->graph_exec = nullptr;
+        g->graph_key = 0;
+    }
+    NGX_CUDA_TRY(cudaFree(g->d_workspace));
+    g->d_workspace = nullptr;
+    g->workspace_bytes = 0;
+    return NGX_OK;
+}
+
+void drop_landmarks(ngx_graph* g) {
+    if (g->d_landmarks != nullptr) {
+        cudaFree(g->d_landmarks);  // waits for the run that used them
+        g->d_landmarks = nullptr;
+        g->landmarks_bytes = 0;
+    }
 }
 
 int grow_buffer(ngx_graph* g, void** buf, size_t* cap, size_t bytes) {
@@ -860,6 +881,10 @@ int ngx_graph_set_stream(ngx_graph* graph, void* stream) {
 int ngx_graph_set_memory_budget(ngx_graph* graph, uint64_t bytes) {
     if (graph == nullptr) {
         return fail(NGX_INVALID_ARGUMENT, "ngx_graph_set_memory_budget: graph is NULL");
+    }
+    if (graph->d_landmarks != nullptr) {
+        NGX_CUDA_TRY(cudaSetDevice(graph->device));
+        drop_landmarks(graph);
     }
     graph->memory_budget = bytes;
     return NGX_OK;

@@ -106,7 +106,8 @@ struct ngx_graph {
     size_t call_out_bytes = 0;
     void* d_call_dag = nullptr;
     size_t call_dag_bytes = 0;
-    // distances from and to the landmarks of a run (2 * kTile * n doubles), computed by each run that uses them
+    // distances from and to the landmarks of a run (2 * kTile * n doubles), computed by each run that uses them. The memory
+    // counts in the budget, stays for the next such run and is given back by the first run without landmarks.
     void* d_landmarks = nullptr;
     size_t landmarks_bytes = 0;
 
@@ -179,11 +180,22 @@ int update_weights_on_device(ngx_graph* g, const double* w);
 
 // Grows the graph's cached workspace to at least `bytes`.
 int ensure_workspace(ngx_graph* g, size_t bytes);
+
+// Gives the cached workspace back.
+int release_workspace(ngx_graph* g);
+
+// Gives the memory of the landmark rows back (allocating and freeing 7 to 51 MB takes 0.7 ms, so runs that use them one
+// after another keep it).
+void drop_landmarks(ngx_graph* g);
+
 // Grows *buf (capacity *cap) to at least `bytes`; contents are not kept. Frees the old buffer only after the stream
 // is idle.
 int grow_buffer(ngx_graph* g, void** buf, size_t* cap, size_t bytes);
 
 // Bytes of device memory a run may use for workspaces (budget, or most of the free memory).
 size_t workspace_budget(const ngx_graph* g);
+
+// What the caller's budget leaves for the workspace (SIZE_MAX without one), whatever memory is free.
+size_t workspace_cap(const ngx_graph* g);
 
 }  // namespace ngx

@@ -321,8 +321,7 @@ int launch_tiles(ngx_graph* g, const ngx_apsp_opts* opts, int tile_mode, const T
     int group = batched && default_shape ? choose_group_size(opts->tile_ctas, resident, num_tiles, resident, typical_n, mean_degree) : 1;
     size_t slot_bytes = data_bytes + group_bytes_of(group);
     int64_t slots = slots_of(group);
-    const size_t kept = g->memory_budget != 0 ? std::min<size_t>(g->workspace_bytes, static_cast<size_t>(g->memory_budget)) : g->workspace_bytes;
-    if (static_cast<size_t>(slots) * slot_bytes > kept) {
+    if (static_cast<size_t>(slots) * slot_bytes > std::min(g->workspace_bytes, workspace_cap(g))) {
         const size_t budget = workspace_budget(g);
         // the group size decides the group storage per slot, which the slot count must leave room for
         const int64_t affordable = static_cast<int64_t>(budget / (data_bytes + group_bytes_of(kMaxGroupSize)));
@@ -696,6 +695,9 @@ int run_sources(ngx_graph* g, const ngx_apsp_opts* opts, int tile_mode, const st
     return launch_tiles(g, opts, tile_mode, job, hist_bins, hist_max, o, extra, ms, true);
 }
 
+// Bytes of the landmarks' distance rows, from and to.
+size_t landmark_bytes(const ngx_graph* g) { return 2 * static_cast<size_t>(kTile) * static_cast<size_t>(g->n) * sizeof(double); }
+
 // Whether a run of `tiles` source tiles pays for landmark bounds: two more tiles, each run by itself, and memory for
 // 2 x kTile rows.
 //  * Twelve waves or more: in fewer, the two extra tiles take as long as they save (two waves' time at 2000 vertices).
@@ -714,15 +716,23 @@ bool landmarks_pay(const ngx_graph* g, const ngx_apsp_opts* opts, int64_t tiles)
     const int64_t resident = 2 * static_cast<int64_t>(g->sm_count);  // the default launch shape
     const int group = choose_group_size(opts->tile_ctas, resident, tiles, resident, static_cast<double>(g->n),
                                         static_cast<double>(g->m_stored) / static_cast<double>(g->n));
-    return tiles >= 12 * (resident / group) && 2 * static_cast<size_t>(kTile) * static_cast<size_t>(g->n) * sizeof(double) <= workspace_budget(g) / 8;
+    return tiles >= 12 * (resident / group) && landmark_bytes(g) <= (workspace_budget(g) + g->landmarks_bytes) / 8;
 }
 
 // Distances from and to kTile landmarks spread over the vertex ids, for the tiles' first bounds (landmark_bounds): one tile
 // over the forward arcs and one over the reverse arcs.
 int compute_landmarks(ngx_graph* g, const ngx_apsp_opts* opts, TileJob* with, float* ms) {
     const size_t rows = static_cast<size_t>(kTile) * static_cast<size_t>(g->n);
-    if (const int rc = grow_buffer(g, &g->d_landmarks, &g->landmarks_bytes, 2 * rows * sizeof(double)); rc != NGX_OK) {
-        return rc;
+    const size_t bytes = landmark_bytes(g);
+    if (g->memory_budget != 0 && g->workspace_bytes + bytes > g->memory_budget) {
+        // the budget holds both only with a smaller workspace, which the runs below allocate
+        if (const int rc = release_workspace(g); rc != NGX_OK) {
+            return rc;
+        }
+    }
+    if (g->d_landmarks == nullptr) {
+        NGX_CUDA_TRY(cudaMalloc(&g->d_landmarks, bytes));
+        g->landmarks_bytes = bytes;
     }
     std::vector<int32_t> landmarks(kTile);
     for (int64_t l = 0; l < kTile; ++l) {
@@ -827,6 +837,10 @@ int run_apsp(ngx_graph* g, const ngx_apsp_opts* caller_opts, ngx_apsp_result* re
         r->cpl = r->efficiency = NAN;  // no reached pairs, as 0 / 0 in AllPairsShortestPath.h:157-158
         return NGX_OK;
     }
+    const bool landmarks = landmarks_pay(g, opts, (num_sources + kTile - 1) / kTile);
+    if (!landmarks) {
+        drop_landmarks(g);
+    }
     const int64_t hist_bins = opts->hist_bins;
     double hist_max = opts->hist_max;
     if (hist_bins > 0 && !(hist_max > 0.0)) {
@@ -837,12 +851,13 @@ int run_apsp(ngx_graph* g, const ngx_apsp_opts* caller_opts, ngx_apsp_result* re
     RunOutputs o;
     float ms = 0.0f;
     TileJob with;
-    if (landmarks_pay(g, opts, (num_sources + kTile - 1) / kTile)) {
+    if (landmarks) {
         const int rc_l = compute_landmarks(g, opts, &with, &ms);
         if (rc_l == NGX_OUT_OF_MEMORY || rc_l == NGX_TIMEOUT) {
             cudaGetLastError();  // the run does without
             set_last_error("");
             with = TileJob{};
+            drop_landmarks(g);
         } else if (rc_l != NGX_OK) {
             return rc_l;
         }

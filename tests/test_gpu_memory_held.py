@@ -1,4 +1,4 @@
-"""Device memory that a handle holds (GPU): arc arrays by the stored arcs, not by the caller's."""
+"""Device memory that a handle holds (GPU): arc arrays by the stored arcs, not by the caller's; landmark rows by the budget."""
 
 from __future__ import annotations
 
@@ -9,6 +9,7 @@ import pytest
 import torch
 
 import neurograph_b200 as ngx
+from neurograph_b200 import synth
 
 pytestmark = pytest.mark.gpu
 
@@ -37,3 +38,22 @@ def test_zero_weights_take_no_arc_memory():
     with ngx.Graph(n, rp, col, w) as g:
         assert held() - before <= 4 * m + 56 * stored + 16 * (n + 1) + SLACK
         assert g.apsp(sources=np.arange(32)).reached_pairs > 0
+
+
+def test_landmark_rows_are_within_the_budget():
+    """A long run over a strongly connected graph of spread lengths starts from landmark rows (512 bytes per vertex, here an
+    eighth of the budget). They are part of what ngx_graph_set_memory_budget caps."""
+    n = 60000
+    budget = 250_000_000  # 14 slots of 17 MB without the rows
+    c = synth.connectome(n, 20, 0.1, weights="lognormal", seed=5, sigma=1.0)
+    with ngx.Graph(c.n, c.row_ptr, c.col, c.w) as g:
+        assert g.scc()["number_components"] == 1
+        sources = g.source_order()[:220 * 32]  # 220 tiles, 18 at a time
+        free = g.apsp(sources=sources, per_source=True, tile_ctas=16)
+    with ngx.Graph(c.n, c.row_ptr, c.col, c.w) as g:  # everything the driver loads with the first run is loaded
+        before = held()
+        g.set_memory_budget(budget)
+        capped = g.apsp(sources=sources, per_source=True, tile_ctas=16)
+        assert held() - before <= budget + SLACK
+    for k, v in free.per_source.items():
+        assert np.array_equal(v, capped.per_source[k]), k
