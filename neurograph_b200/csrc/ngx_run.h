@@ -69,13 +69,15 @@ int prepare_sources(const ngx_graph* g, const ngx_apsp_opts* opts, std::vector<i
 // (few arcs per bucket: a narrow one runs many nearly empty phases).
 double degree_delta_scale(int64_t n, int64_t m);
 // Bucket width of the batched form when the caller gives none: twice that where wide buckets re-relax little, which is on
-// sparse graphs (mean out-degree below 32) and where few arcs are much shorter than the mean (mean(len) x mean(1 / len)
+// sparse graphs (mean out-degree below 28) and where few arcs are much shorter than the mean (mean(len) x mean(1 / len)
 // below 2: 1 for equal lengths, 1.3 and 2.7 for log-normal weights of sigma 0.5 and 1, 1.6 for integers up to 10). Kernel
 // times in ms at 1 x and 2 x the width by density:
 //   sigma 0.5: APSP of 2048 sources, n = 5e4, degree 40: 27.0, 25.8; gradient of the same 57.7, 56.2; Brandes, 3e4, 25: 39.1, 36.6;
 //   integers: Brandes, n = 5000, degree 6: 13.2, 12.7; 1e4, 40: 59.5, 59.2; APSP, 3000, 50: 2.03, 2.04; unit weights equal;
 //   sigma 1, sparse: APSP, n = 300, degree 8: 0.45, 0.37; 2e4, 2: 33.1, 29.8; 5e4, 6: 25.1, 24.1; Brandes, 3e4, 12: 42.3, 39.8;
-//   the line: sigma 1, Brandes, n = 2e5, degree 30: 40.4, 40.1; APSP, 3e4, 60: 37.5, 37.8; 1e4, 90: 32.1, 32.7.
+//   the line, sigma 1, Brandes at degrees 20, 24, 28 and 31: n = 8000: 20.5, 20.6; 21.4, 21.4; 21.1, 21.6; 21.5, 21.7;
+//   3e4: 40.2, 39.0; 39.6, 39.4; 39.9, 40.0; 40.8, 40.7; 2e5: 39.4, 38.2; 36.9, 35.6; 37.1, 36.4; 37.8, 37.1 (larger graphs
+//   would have it higher); above it: APSP, 3e4, 60: 37.5, 37.8; 1e4, 90: 32.1, 32.7.
 double default_delta_scale(const GraphPart& part);
 double pick_delta(double mean_len, double requested, double scale);
 int alloc_outputs(ngx_graph* g, int64_t num_graphs, int64_t num_sources, int64_t hist_bins, bool want_rows, RunOutputs& o, bool persistent);

@@ -62,7 +62,7 @@ double degree_delta_scale(int64_t n, int64_t m) {
 
 double default_delta_scale(const GraphPart& part) {
     const double spread = part.mean_len_regular * part.mean_len_inverse;  // the same for both metrics
-    const bool wide = part.m_stored < 32 * part.n || spread < 2.0;
+    const bool wide = part.m_stored < 28 * part.n || spread < 2.0;
     return (wide ? 2.0 : 1.0) * degree_delta_scale(part.n, part.m_stored);
 }
 

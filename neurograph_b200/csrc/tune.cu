@@ -79,7 +79,7 @@ int ngx_graph_autotune(ngx_graph* g, int task, int64_t sample_sources, ngx_tunin
         const int64_t wave = static_cast<int64_t>(g->sm_count) * 2 * kTile;
         const int64_t k = std::min<int64_t>(g->n, sample_sources > 0 ? sample_sources : wave);
         if (k == 0) {
-            t.delta_scale = degree_delta_scale(g->parts[0].n, g->parts[0].m_stored);
+            t.delta_scale = default_delta_scale(g->parts[0]);
             t.block_threads = 512;
             t.ctas_per_sm = 2;
             t.tile_ctas = 1;
@@ -90,9 +90,14 @@ int ngx_graph_autotune(ngx_graph* g, int task, int64_t sample_sources, ngx_tunin
         }
         const std::vector<int64_t> sources(g->source_order.begin(), g->source_order.begin() + k);
         const double mean = g->parts[0].mean_len_regular;
-        // bucket widths: the width by the graph's degree first, then fixed multiples of the mean length (2 x, which sparse
-        // graphs and little spread want, among them)
-        const double kScales[] = { degree_delta_scale(g->parts[0].n, g->parts[0].m_stored), 0.125, 0.25, 0.5, 1.0, 2.0 };
+        // bucket widths: the one untuned runs use first, the width by the graph's degree where that is another, then fixed
+        // multiples of the mean length
+        std::vector<double> scales = { default_delta_scale(g->parts[0]) };
+        for (const double sc : { degree_delta_scale(g->parts[0].n, g->parts[0].m_stored), 0.125, 0.25, 0.5, 1.0, 2.0 }) {
+            if (sc != scales[0]) {
+                scales.push_back(sc);
+            }
+        }
         static const Shape kShapes[] = { { 512, 2 }, { 384, 2 }, { 256, 3 }, { 256, 4 } };
         const int tiles = static_cast<int>((k + kTile - 1) / kTile);
         // CTAs per tile: the library's own choice (0: the bucket-width trials run with it, as untuned runs do), 1, 2,
@@ -111,7 +116,7 @@ int ngx_graph_autotune(ngx_graph* g, int task, int64_t sample_sources, ngx_tunin
         int tile_ctas = 0;
         int trials = 0;
         // one parameter at a time: bucket width, then block shape, then CTAs per tile
-        for (const double sc : kScales) {
+        for (const double sc : scales) {
             double rate = 0.0;
             if (const int rc = trial(g, task, sources, pick_delta(mean, 0.0, sc), shape, tile_ctas, &rate); rc != NGX_OK) {
                 return rc;
