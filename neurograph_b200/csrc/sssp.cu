@@ -700,7 +700,13 @@ size_t landmark_bytes(const ngx_graph* g) { return 2 * static_cast<size_t>(kTile
 
 // Whether a run of `tiles` source tiles pays for landmark bounds: two more tiles, each run by itself, and memory for
 // 2 x kTile rows.
-//  * Twelve waves or more: in fewer, the two extra tiles take as long as they save (two waves' time at 2000 vertices).
+//  * Twelve waves or more of the library's own group size. Kernel times without and with at the line (log-normal lengths of
+//    sigma 1, APSP; Brandes; gradient, ms): 14,000 vertices at degree 40, 256 tiles: 30.6, 29.4; 39.1, 38.4; 57.6, 56.8; 20,000
+//    at 60, 256 tiles: 48.5, 44.0; 59.4, 56.1; 90.3, 86.8; 30,000 at 40, 168 tiles: 44.5, 42.0; 55.5, 54.0; 85.6, 84.5; 100,000
+//    at 100, 96 tiles: 110.5, 99.4; 132.4, 123.9; 203.4, 195.7; 200,000 at 60, 60 tiles: 124.8, 119.8; 154.6, 149.5; 255.4, 248.8.
+//  * 128 tiles or more where the caller sets the group size, since waves of any size say little about a tile's work: with 74
+//    CTAs (12 waves are 48 tiles) APSP without and with, 30,000 at 40: 48 tiles 17.5, 18.2; 64: 23.4, 23.7; 96: 34.8, 34.7; 128:
+//    46.7, 45.7; 8000 at 40: 48: 9.2, 9.9; 96: 18.2, 18.6; 128: 24.3, 24.4; 160: 30.7, 29.9.
 //  * Lengths that spread: mean(len) x mean(1 / len) is 1 for equal lengths, 1.3 and 2.7 for log-normal weights of sigma 0.5
 //    and 1, 1.6 for integers up to 10. Measured kernel times without and with: sigma 1, APSP of 148 tiles on 100,000
 //    vertices 181 and 158 ms, Brandes of 74 tiles 108 and 102 ms, APSP of 938 tiles on 30,000 vertices 267 and 240 ms;
@@ -716,7 +722,7 @@ bool landmarks_pay(const ngx_graph* g, const ngx_apsp_opts* opts, int64_t tiles)
     const int64_t resident = 2 * static_cast<int64_t>(g->sm_count);  // the default launch shape
     const int group = choose_group_size(opts->tile_ctas, resident, tiles, resident, static_cast<double>(g->n),
                                         static_cast<double>(g->m_stored) / static_cast<double>(g->n));
-    return tiles >= 12 * (resident / group) && landmark_bytes(g) <= (workspace_budget(g) + g->landmarks_bytes) / 8;
+    return tiles >= 12 * (resident / group) && (opts->tile_ctas == 0 || tiles >= 128) && landmark_bytes(g) <= (workspace_budget(g) + g->landmarks_bytes) / 8;
 }
 
 // Distances from and to kTile landmarks spread over the vertex ids, for the tiles' first bounds (landmark_bounds): one tile
