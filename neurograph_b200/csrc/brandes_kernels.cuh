@@ -38,12 +38,11 @@ struct BrandesParams {
     int32_t* ws_loff;               // slots * (n + 2): start of each level in ws_list
     uint32_t* ws_scnt;              // slots * n * kTile: DAG successors per (vertex, source), then fill positions
     uint32_t* ws_soff;              // slots * (n * kTile + 1): start of each (vertex, source)'s successor list
-    uint32_t* ws_succ;              // slots * succ_capacity: successor lists (indices into the forward CSR)
+    uint32_t* ws_succ;              // slots * succ_capacity: successor lists (targets; the adjoint of tied tiles: forward-CSR indices)
     int64_t succ_capacity;          // entries per slot; a tile with more DAG arcs uses the arc-scanning passes
     unsigned long long* bc;         // 2 * n fixed point (Brandes), or nullptr
     unsigned long long* grad_cpl;   // 2 * m_user fixed point (adjoint), or nullptr
     unsigned long long* grad_eff;   // 2 * m_user fixed point (adjoint), or nullptr
-    unsigned long long* levels;     // unused (levels are counted in the run counters)
     int* sigma_inexact;             // set when a pushed sigma sum reaches 2^53 (the host then reruns in pull form)
     int sigma_pull;                 // 1: pull form for sigma
 };
@@ -304,8 +303,8 @@ __device__ __forceinline__ void brandes_delta_vertex(const DeviceCsr& g, int v, 
 // The DAG of a tile is about one arc per (vertex, source) without ties, against deg arcs scanned per (vertex, source)
 // by the arc-scanning passes. The count pass (dag_count: warp per vertex, lane per source, coalesced distance rows) visits
 // every DAG arc; it also counts successors per (vertex, source). A group-wide prefix sum gives each (vertex, source) its
-// list, a second pass (dag_fill) fills the lists (forward-CSR arc indices), and each list is sorted so that every sum
-// over it has a fixed order. sigma and delta then touch only DAG arcs.
+// list, a second pass (dag_fill) fills the lists, and each list is sorted so that every sum over it has a fixed order. sigma
+// and delta then touch only DAG arcs.
 
 // Sorts each successor list by its entries (the fill order depends on timing; the sums must not). Lists are spread
 // over the threads of the group: thread `first` of `stride` takes lists first, first + stride, ...
@@ -432,10 +431,10 @@ __device__ __forceinline__ void dag_sigma_level(const DeviceCsr& g, const int32_
     }
 }
 
-// One level of the sigma pass when the tile's DAGs are trees: every successor gets sigma 1 and joins the next level.
-template <bool kTarget>
-__device__ __forceinline__ void dag_tree_level(const DeviceCsr& g, const int32_t* entries, int len, double* sigma, const uint32_t* soff,
-                                               const uint32_t* succ, int32_t* next_list, int* next_len, int lane, int warp, int nwarps) {
+// One level of the adjoint's forward pass when the tile's DAGs are trees: every path count is 1 (nothing reads it), and every
+// successor joins the next level. The lists hold targets.
+__device__ __forceinline__ void dag_tree_level(const int32_t* entries, int len, const uint32_t* soff, const uint32_t* succ, int32_t* next_list,
+                                               int* next_len, int lane, int warp, int nwarps) {
     for (int base = warp * 32; base < len; base += nwarps * 32) {
         const int i = base + lane;
         uint32_t entry = 0, beg = 0, count = 0;
@@ -463,17 +462,12 @@ __device__ __forceinline__ void dag_tree_level(const DeviceCsr& g, const int32_t
                 const int owner = pair_owner(off, ok[u] ? q : 0u);
                 const uint32_t j = __shfl_sync(0xFFFFFFFFu, beg, owner) + (q - __shfl_sync(0xFFFFFFFFu, off, owner));
                 sx[u] = __shfl_sync(0xFFFFFFFFu, entry, owner) & 31u;
-                x[u] = 0;
-                if (ok[u]) {
-                    const uint32_t e = __ldcg(&succ[j]);
-                    x[u] = kTarget ? e : static_cast<uint32_t>(ldg_arc(&g.arcs[e]).col);
-                }
+                x[u] = ok[u] ? __ldcg(&succ[j]) : 0u;
             }
 #pragma unroll
             for (int u = 0; u < kLevelUnroll; ++u) {
                 const uint32_t q = p0 + static_cast<uint32_t>(u * 32 + lane);
                 if (ok[u]) {
-                    sigma[static_cast<int64_t>(x[u]) * kTile + sx[u]] = 1.0;
                     next_list[at + static_cast<int>(q)] = static_cast<int32_t>((x[u] << 5) | sx[u]);
                 }
             }
@@ -483,7 +477,8 @@ __device__ __forceinline__ void dag_tree_level(const DeviceCsr& g, const int32_t
 
 // delta (and the adjoint terms) over one level: each entry pulls over its sorted successor list. Pair contributions
 // go through the warp's slice of `buf` (32 values per unrolled pair, twice for the adjoint) and each entry's lane adds
-// its own in list order, so every sum runs in the same order as a sequential loop over the list.
+// its own in list order, so every sum runs in the same order as a sequential loop over the list. kTree: the adjoint on
+// tree tiles (betweenness walks those, dag_tree_walk).
 template <int kMode, bool kTree>
 __device__ __forceinline__ void dag_delta_level(const DeviceCsr& g, const int32_t* entries, int len, const unsigned long long* dist, const double* sigma,
                                                 double* delta, double* delta_g, const uint32_t* soff, const uint32_t* succ, unsigned long long* grad_cpl,

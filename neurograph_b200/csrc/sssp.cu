@@ -426,7 +426,6 @@ int launch_tiles(ngx_graph* g, const ngx_apsp_opts* opts, int tile_mode, const T
             bp.bc = extra->bc;
             bp.grad_cpl = extra->grad_cpl;
             bp.grad_eff = extra->grad_eff;
-            bp.levels = extra->levels;
             bp.sigma_inexact = extra->sigma_inexact;
             bp.sigma_pull = extra->sigma_pull;
         }

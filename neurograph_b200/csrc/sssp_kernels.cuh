@@ -8,8 +8,9 @@
 //   near phase   vertices whose pending (vertex, source) pairs lie below theta are expanded; an improvement below
 //                theta marks the pair pending for the next iteration, one at or above theta marks it "far"; after
 //                the iteration the next queue is compacted from the pending masks (warp ballot + prefix);
-//   bucket step  when no near work is left, one pass over the far marks finds the smallest pending distance d_min,
-//                theta becomes (floor(d_min / delta) + 1) * delta, and the pairs below it move to the near queue.
+//   bucket step  when no near work is left, theta becomes (floor(d_min / delta) + 1) * delta, where d_min, the smallest
+//                pending distance, was gathered by the relaxations that set far marks; one pass over the marks then moves
+//                the pairs below theta to the near queue and finds the smallest that stays.
 // Relaxation is fl(d[u] + len) compared and stored with a 64-bit atomicMin on the bit pattern, which orders
 // non-negative doubles like their values. The label-correcting fixed point is the same as the reference Dijkstra's
 // (PriorityQueueVariant.h:47-93: d[v] = min over arcs of fl(d[u] + |w|)), so distances are bit-identical.
@@ -245,9 +246,9 @@ struct ExpandArgs {
     int small_entries;
 };
 
-// Dynamic shared memory of the tile kernel, before the histogram. The distance phase's warp scratch overlays the
-// epilogue's accumulators (2 x kTile x kAccDigits words, zero outside the distance phase) and, after them, the scan
-// partials of the DAG phase.
+// Dynamic shared memory of the tile kernel, before the histogram. The warp scratch of the distance phase and of the DAG
+// passes overlays the epilogue's accumulators (2 x kTile x kAccDigits words, which the epilogue zeroes first) and, after
+// them, the scan partials of the DAG phase.
 struct __align__(16) TileSmem {
     WarpScratch warp[kMaxWarps];
     WarpWork work[kMaxWarps];
@@ -1220,7 +1221,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
                 break;
             }
             if (use_lists) {
-                if (kMode == kModeBrandes || tree) {
+                if (kMode == kModeBrandes || tree) {  // (targets only)
                     dag_fill<true>(b.arc_src, low, cnt, pred, soff, scnt, succ, NGX_GW);
                 } else {
                     dag_fill<false>(b.arc_src, low, cnt, pred, soff, scnt, succ, NGX_GW);
@@ -1294,9 +1295,9 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
                     break;
                 }
                 const unsigned level = s.level;
-                if (tree) {
-                    dag_tree_level<true>(g, list + start, len, sigma, soff, succ, list + start + len, &ctl()->next_len, lane, NGX_GW,
-                                                          NGX_GWARPS);
+                // (tree tiles of betweenness took the walk above)
+                if (kMode == kModeGrad && tree) {
+                    dag_tree_level(list + start, len, soff, succ, list + start + len, &ctl()->next_len, lane, NGX_GW, NGX_GWARPS);
                 } else {
                     dag_sigma_level<kMode == kModeBrandes>(g, list + start, len, sigma, cnt, soff, succ, list + start + len, &ctl()->next_len,
                                                            b.sigma_inexact, lane, NGX_GW, NGX_GWARPS);
@@ -1342,8 +1343,8 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
             for (int level = levels - 1; level >= lowest; --level) {
                 const int start = __ldcg(&loff[level]);
                 const int end = __ldcg(&loff[level + 1]);
-                if (tree) {
-                    dag_delta_level<kMode, true>(g, list + start, end - start, dist, sigma, delta, delta_g, soff, succ, b.grad_cpl, b.grad_eff,
+                if (kMode == kModeGrad && tree) {
+                    dag_delta_level<kModeGrad, true>(g, list + start, end - start, dist, sigma, delta, delta_g, soff, succ, b.grad_cpl, b.grad_eff,
                                                  reinterpret_cast<double*>(s_acc_sum), lane, warp, NGX_GW, NGX_GWARPS);
                 } else {
                     dag_delta_level<kMode, false>(g, list + start, end - start, dist, sigma, delta, delta_g, soff, succ, b.grad_cpl, b.grad_eff,
