@@ -582,39 +582,37 @@ __device__ __forceinline__ void dag_delta_level(const DeviceCsr& g, const int32_
 }
 
 // Adds each active lane's terms c (a whole number) and cg to the gradients of its arc e, in 128-bit fixed point. The
-// sources of a tile are near one another, so most lanes of a vertex share its predecessor arc: the lanes of one arc are
-// summed first (exactly: integer adds), and one lane per arc adds the sums, a third of the atomics at out-degree 40.
+// sources of a tile are near one another, so most lanes of a vertex share its predecessor arc: one lane per arc adds the
+// sums of its lanes (exact integer adds, in any order), a third of the atomics at out-degree 40.
+// The lanes of an arc form a list, each pointing at the next higher one, and are summed by list ranking (pointer jumping,
+// Wyllie 1979): in each step a lane adds what the lane it points at has gathered and then points where that one points, so
+// after k steps it holds the next 2^k lanes of its list and at most five steps serve every list of the warp.
 __device__ __forceinline__ void add_arc_terms(const Arc* arcs, bool active, uint32_t e, double c, double cg, int lane, unsigned long long* grad_cpl,
                                               unsigned long long* grad_eff) {
-    const unsigned act = __ballot_sync(0xFFFFFFFFu, active);
-    if (!active) {
-        return;
-    }
-    unsigned long long sum = static_cast<unsigned long long>(c);
+    constexpr unsigned kAll = 0xFFFFFFFFu;
+    // lanes without a term (e = 0xFFFFFFFF, no arc's index) form a list of zeros of their own
+    const unsigned list = __match_any_sync(kAll, active ? e : kAll);
+    unsigned long long whole = active ? static_cast<unsigned long long>(c) : 0ull;
     unsigned long long lo, hi;
-    fixed_parts(cg, lo, hi);
-    const unsigned all = __match_any_sync(act, e);
-    unsigned peers = all & (0xFFFFFFFEu << lane);  // the arc's lanes above this one
-    int rank = __popc(all & lanemask_lt());
-    while (__any_sync(act, peers != 0u)) {
-        const int next = __ffs(peers);
-        const int from = next != 0 ? next - 1 : lane;
-        const unsigned long long o_sum = __shfl_sync(act, sum, from);
-        const unsigned long long o_lo = __shfl_sync(act, lo, from);
-        const unsigned long long o_hi = __shfl_sync(act, hi, from);
-        if (next != 0) {
-            sum += o_sum;
-            const unsigned long long t = lo + o_lo;
-            hi += o_hi + (t < lo ? 1ull : 0ull);
-            lo = t;
+    fixed_parts(active ? cg : 0.0, lo, hi);
+    const unsigned above = list & ~lanemask_lt() & ~(1u << lane);
+    int next = above != 0u ? __ffs(above) - 1 : 32;  // 32: the end of the list
+    while (__any_sync(kAll, next < 32)) {
+        const int from = next & 31;
+        const unsigned long long whole_n = __shfl_sync(kAll, whole, from);
+        const unsigned long long lo_n = __shfl_sync(kAll, lo, from);
+        const unsigned long long hi_n = __shfl_sync(kAll, hi, from);
+        const int next_n = __shfl_sync(kAll, next, from);
+        if (next < 32) {
+            whole += whole_n;
+            lo += lo_n;
+            hi += hi_n + (lo < lo_n ? 1ull : 0ull);
+            next = next_n;
         }
-        // lanes of odd rank have been added to the one below and drop out
-        peers &= __ballot_sync(act, (rank & 1) == 0);
-        rank >>= 1;
     }
-    if (lane == __ffs(all) - 1) {
+    if (active && (list & lanemask_lt()) == 0u) {  // the head of its list
         const int64_t id = ldg_arc(&arcs[e]).id;
-        atomicAdd(&grad_cpl[2 * id + 1], sum);
+        atomicAdd(&grad_cpl[2 * id + 1], whole);
         if ((lo | hi) != 0ull) {
             fixed_add_parts(&grad_eff[2 * id], lo, hi);
         }
