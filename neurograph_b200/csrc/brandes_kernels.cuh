@@ -431,10 +431,11 @@ __device__ __forceinline__ void dag_sigma_level(const DeviceCsr& g, const int32_
     }
 }
 
-// One level of the adjoint's forward pass when the tile's DAGs are trees: every path count is 1 (nothing reads it), and every
-// successor joins the next level. The lists hold targets.
-__device__ __forceinline__ void dag_tree_level(const int32_t* entries, int len, const uint32_t* soff, const uint32_t* succ, int32_t* next_list,
-                                               int* next_len, int lane, int warp, int nwarps) {
+// One level of the adjoint's forward pass when the tile's DAGs are trees: every path count is 1, and every successor joins the
+// next level. The lists hold targets. (No later pass reads these counts; without the store the compiler allocates the tile
+// kernel's registers so that the distance phase takes 7 to 11 % longer, 79.0 instead of 77.2 ms for a gradient on 10,007 vertices.)
+__device__ __forceinline__ void dag_tree_level(const int32_t* entries, int len, double* sigma, const uint32_t* soff, const uint32_t* succ,
+                                               int32_t* next_list, int* next_len, int lane, int warp, int nwarps) {
     for (int base = warp * 32; base < len; base += nwarps * 32) {
         const int i = base + lane;
         uint32_t entry = 0, beg = 0, count = 0;
@@ -468,6 +469,7 @@ __device__ __forceinline__ void dag_tree_level(const int32_t* entries, int len, 
             for (int u = 0; u < kLevelUnroll; ++u) {
                 const uint32_t q = p0 + static_cast<uint32_t>(u * 32 + lane);
                 if (ok[u]) {
+                    sigma[static_cast<int64_t>(x[u]) * kTile + sx[u]] = 1.0;
                     next_list[at + static_cast<int>(q)] = static_cast<int32_t>((x[u] << 5) | sx[u]);
                 }
             }

@@ -1297,7 +1297,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) tile_kernel(const __grid_c
                 const unsigned level = s.level;
                 // (tree tiles of betweenness took the walk above)
                 if (kMode == kModeGrad && tree) {
-                    dag_tree_level(list + start, len, soff, succ, list + start + len, &ctl()->next_len, lane, NGX_GW, NGX_GWARPS);
+                    dag_tree_level(list + start, len, sigma, soff, succ, list + start + len, &ctl()->next_len, lane, NGX_GW, NGX_GWARPS);
                 } else {
                     dag_sigma_level<kMode == kModeBrandes>(g, list + start, len, sigma, cnt, soff, succ, list + start + len, &ctl()->next_len,
                                                            b.sigma_inexact, lane, NGX_GW, NGX_GWARPS);
