@@ -207,8 +207,11 @@ const void* tile_kernel_for_block(int block, int ctas_per_sm, bool reach, bool m
 //    0.6 sqrt(n) (n = 2e4, 2 tiles: 37: 1.22, 74: 0.94, 148: 1.05 ms; n = 300, 10 tiles: 4: 0.49, 8-29: 0.45). At least
 //    four tiles stay in flight.
 //  * Sparse graphs (mean out-degree below 4) have long shortest paths, so many phases with few entries each: one CTA per
-//    tile while there are two tiles for every resident CTA (n = 2e4, degree 2, 626 tiles: 1: 70, 3: 75, 7: 92, 14: 118 ms),
-//    more in proportion when there are fewer.
+//    tile while there are two tiles for every resident CTA, more in proportion when there are fewer. Right at n = 2e4 and
+//    degree 2 (626 tiles, APSP: 1: 65, 2: 66, 4: 71, 16: 109 ms) and with few tiles (n = 1e5, degree 3, 94 tiles, the rule's 6:
+//    46, 8-16: 47, 1: 86); larger graphs and degrees near 4 with many tiles would be faster with 4 to 16: n = 2e4, degree 3.9: 1:
+//    85, 4: 76; n = 6e4, degree 2: 1: 561, 4: 552; n = 1e5, degree 3, 500 tiles: 1: 320, the rule's 323, 8: 251; n = 3e5, degree
+//    3.9, 313 tiles: the rule's 715, 16: 465 (four tiles in L2, the rule before this one: 112, 1391, 601 and 878 ms).
 //  * Memory: when the device affords fewer workspace slots than that, each slot gets enough CTAs to use every SM.
 int choose_group_size(int requested, int64_t resident, int64_t num_tiles, int64_t affordable_slots, double typical_n, double mean_degree) {
     if (requested > 0) {

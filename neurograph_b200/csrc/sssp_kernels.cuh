@@ -428,8 +428,8 @@ constexpr int kPackPairs = 64;
 // Expands a group of m small queue entries together: w.rank[t], t < ktot <= 32, names the t-th (entry, pending source) of
 // the group. Lane t takes it and walks its entry's arcs, kUnroll at a time: the lanes of an entry read the same arc
 // records and neighbouring distances of the same rows, no lane needs to find its pairs, and the group takes as long as
-// its entry with the most arcs. The relaxations and the counters are batched_expand's; the arcs are not filtered (a bound read per arc would cost as much as the few distance reads it
-// saves).
+// its entry with the most arcs. The relaxations and the counters are batched_expand's; the arcs are not filtered (a bound
+// read per arc would cost as much as the few distance reads it saves).
 template <int kUnroll, bool kReach>
 __device__ __forceinline__ void packed_expand(TileSmem& sh, WarpScratch& w, WarpWork& work, int m, int ktot, int lane,
                                               unsigned long long& far_min) {
