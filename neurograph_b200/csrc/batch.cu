@@ -223,6 +223,10 @@ int ngx_batch_run(ngx_graph* g, const ngx_batch_opts* opts, ngx_apsp_result* res
         }
         NGX_CUDA_TRY(cudaSetDevice(g->device));
         *g->h_abort = 0;
+        // a batch of one graph is built on the device, which leaves the order of its sources to the first run
+        if (const int rc = ensure_source_order(g); rc != NGX_OK) {
+            return rc;
+        }
         ngx_apsp_opts aopts{};
         aopts.metric = opts->metric;
         aopts.mode = NGX_MODE_BATCHED;
@@ -421,6 +425,9 @@ int ngx_batch_autotune(ngx_graph* g, int task, double* class_scales) {
         }
         NGX_CUDA_TRY(cudaSetDevice(g->device));
         *g->h_abort = 0;
+        if (const int rc = ensure_source_order(g); rc != NGX_OK) {
+            return rc;
+        }
         static const double kScales[] = { 0.125, 0.25, 0.5, 1.0, 2.0, 4.0 };
         g->tuned[mode] = ngx_tuning{};
         // the graph of each size class whose first wave is timed: its median-size member

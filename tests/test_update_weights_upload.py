@@ -29,6 +29,7 @@ static size_t fail_size = 0;      /* the next host-to-device copy of this size f
 static int copies_of_size = 0;    /* host-to-device copies of the watched size that succeeded */
 static size_t watched = 0;
 void fake_fail_copy(size_t bytes) { fail_size = bytes; watched = bytes; copies_of_size = 0; }
+void fake_watch_copy(size_t bytes) { watched = bytes; copies_of_size = 0; }
 int fake_copies(void) { return copies_of_size; }
 err cudaMalloc(void** p, size_t n) { *p = calloc(1, n ? n : 1); return *p ? 0 : 2; }
 err cudaFree(void* p) { free(p); return 0; }
@@ -50,6 +51,7 @@ err cudaGetDevice(int* d) { *d = 0; return 0; }
 err cudaDeviceGetAttribute(int* v, int attr, int dev) { (void)dev; *v = attr == 75 ? 10 : 148; return 0; }
 err cudaStreamCreateWithFlags(void** s, unsigned f) { (void)f; *s = NULL; return 0; }
 err cudaMemGetInfo(size_t* f, size_t* t) { *f = *t = (size_t)1 << 36; return 0; }
+err cudaFuncGetAttributes(int* attr, const void* f) { (void)f; memset(attr, 0, 64); attr[6] = 1024; attr[8] = attr[9] = 100; return 0; }
 const char* cudaGetErrorString(err e) { (void)e; return "fake error"; }
 void** __cudaRegisterFatBinary(void* f) { static void* h; (void)f; return &h; }
 """
