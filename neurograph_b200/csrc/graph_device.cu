@@ -251,7 +251,8 @@ int build_graph_on_device(const ngx_csr* csr, ngx_graph* g) {
     } joiner{ sums_thread };
 
     // three blocks: what is needed to count the stored arcs, and, once they are counted (zero weights are not stored), the
-    // handle's arrays and the sort's
+    // sort's and the handle's arrays (in this order: with the arrays first, runs on 300 vertices took 2 % longer, 0.385 and
+    // 0.376 ms of kernel time, by where the arrays then lay)
     const size_t mu = static_cast<size_t>(m_user);
     int64_t* d_user_rows = nullptr;
     int32_t* d_col = nullptr;
@@ -299,17 +300,6 @@ int build_graph_on_device(const ngx_csr* csr, ngx_graph* g) {
     }
 
     const size_t ms = static_cast<size_t>(m);
-    Carver arrays;
-    arrays.take(&g->d_row_ptr, static_cast<size_t>(n) + 1);
-    arrays.take(&g->d_rrow_ptr, static_cast<size_t>(n) + 1);
-    arrays.take(&g->d_arcs_regular, ms);
-    arrays.take(&g->d_arcs_inverse, ms);
-    arrays.take(&g->d_rarcs, ms);
-    arrays.take(&g->d_arc_src, ms);
-    arrays.take(&g->d_stored_of_user, mu);
-    if (const int rc = arrays.allocate(&g->d_block); rc != NGX_OK) {
-        return rc;
-    }
     uint32_t *d_target = nullptr, *d_target_sorted = nullptr;  // unsigned keys: the sort looks at the low bits only
     int32_t *d_index = nullptr, *d_index_sorted = nullptr;
     char* d_sort = nullptr;
@@ -323,6 +313,17 @@ int build_graph_on_device(const ngx_csr* csr, ngx_graph* g) {
     sort_temps.take(&d_index_sorted, ms);
     sort_temps.take(&d_sort, sort_bytes);
     if (const int rc = sort_temps.allocate(&sort_tmp.p); rc != NGX_OK) {
+        return rc;
+    }
+    Carver arrays;
+    arrays.take(&g->d_row_ptr, static_cast<size_t>(n) + 1);
+    arrays.take(&g->d_rrow_ptr, static_cast<size_t>(n) + 1);
+    arrays.take(&g->d_arcs_regular, ms);
+    arrays.take(&g->d_arcs_inverse, ms);
+    arrays.take(&g->d_rarcs, ms);
+    arrays.take(&g->d_arc_src, ms);
+    arrays.take(&g->d_stored_of_user, mu);
+    if (const int rc = arrays.allocate(&g->d_block); rc != NGX_OK) {
         return rc;
     }
     NGX_CUDA_TRY(cudaMemcpyAsync(g->d_row_ptr, d_rows, (static_cast<size_t>(n) + 1) * 8, cudaMemcpyDeviceToDevice, s));
