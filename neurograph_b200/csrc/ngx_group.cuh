@@ -68,8 +68,8 @@ struct Group {
     // control block into `local` (its shared memory). bar_target is the CTA's count of barriers passed (shared). A
     // CTA that gave up waiting is out of the group for the rest of the launch: its bar_target becomes kGroupLeft, it
     // joins no later barrier, and its local control block is halted (Ctl::halt: no work left). What the CTAs do between
-    // this barrier and the next may stay undone from then on, so it must leave its loops here and end, without a look at the
-    // group's state; the others give up at the next barrier. The run then reports NGX_TIMEOUT.
+    // this barrier and the next may stay undone from then on, so it must leave its loops here, and follow no pointer or list
+    // of the group's state; the others give up at the next barrier. The run then reports NGX_TIMEOUT.
     template <typename Update>
     __device__ __forceinline__ void sync(Ctl& local, unsigned& bar_target, Update&& update) const {
         __syncthreads();
