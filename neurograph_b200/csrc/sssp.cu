@@ -702,10 +702,12 @@ size_t landmark_bytes(const ngx_graph* g) { return 2 * static_cast<size_t>(kTile
 
 // Whether a run of `tiles` source tiles pays for landmark bounds: two more tiles, each run by itself, and memory for
 // 2 x kTile rows.
-//  * Twelve waves or more of the library's own group size. Kernel times without and with at the line (log-normal lengths of
-//    sigma 1, APSP; Brandes; gradient, ms): 14,000 vertices at degree 40, 256 tiles: 30.6, 29.4; 39.1, 38.4; 57.6, 56.8; 20,000
-//    at 60, 256 tiles: 48.5, 44.0; 59.4, 56.1; 90.3, 86.8; 30,000 at 40, 168 tiles: 44.5, 42.0; 55.5, 54.0; 85.6, 84.5; 100,000
-//    at 100, 96 tiles: 110.5, 99.4; 132.4, 123.9; 203.4, 195.7; 200,000 at 60, 60 tiles: 124.8, 119.8; 154.6, 149.5; 255.4, 248.8.
+//  * Twelve waves or more of the library's own group size. Kernel times without and with at that line, log-normal lengths of
+//    sigma 1 (APSP; Brandes; gradient, ms): 14,000 vertices at degree 40, 252 tiles: 30.7, 29.6; 39.1, 38.0; 58.0, 57.1; 20,000
+//    at 60, 252: 47.5, 43.7; 58.5, 55.3; 88.7, 85.6; 30,000 at 40, 168: 45.1, 42.9; 55.5, 54.5; 86.8, 85.2; 50,000 at 40, 96: 44.6,
+//    43.8; 55.0, 55.5; 85.2, 84.9; 100,000 at 40, 60: 57.2, 58.8; 71.4, 72.0; 113.5, 114.1 (the one graph that would have the line
+//    higher, at 75 tiles); 100,000 at 100, 60: 69.9, 64.4; 84.6, 81.4; 128.8, 125.2; 200,000 at 40, 48: 93.9, 93.0; 118.7, 118.6;
+//    194.7, 194.0; 1,000,000 at 40, 48: 527, 500; 661, 644; 1127, 1108.
 //  * 128 tiles or more where the caller sets the group size, since waves of any size say little about a tile's work: with 74
 //    CTAs (12 waves are 48 tiles) APSP without and with, 30,000 at 40: 48 tiles 17.5, 18.2; 64: 23.4, 23.7; 96: 34.8, 34.7; 128:
 //    46.7, 45.7; 8000 at 40: 48: 9.2, 9.9; 96: 18.2, 18.6; 128: 24.3, 24.4; 160: 30.7, 29.9.
